@@ -53,6 +53,7 @@
 
 #include "common.cuh"
 #include "kernels.hpp"
+#include "sine_solve.cuh"
 #include "spmv.cuh"
 
 namespace cup2d {
@@ -80,26 +81,30 @@ static_assert(Q_SUMB + 1 <= kRedQ, "reduction slots");
 static_assert(Q_MX + 1 <= kRedQMean, "reduction slots (mean constraint)");
 
 // Shared memory of the solve kernels, per precision T of the Krylov vectors:
-// P^-1, the P^-1 staging tiles, the staged SpMV rings and the reduction
-// scratch.  Both layouts stay below 54 KB so that the kernels run at 3 CTAs
-// per SM (the FP64 batch and the server's instances) within the 164 KB
-// shared carve-out and leave 92 KB of the unified L1/shared array as L1
-// (their spill reloads and table reads live there: the same kernel with the
-// whole array given to shared memory ran 11 % slower).  The kernels at 2
-// CTAs per SM take a smaller carve-out and keep more L1.
+// per warp one ring of the staged SpMV, which also serves as the scratch of
+// the block solves' transposes and of the register-path SpMV, and the
+// reduction scratch.
 template <class T>
-union TileSmem;
-template <>
-union TileSmem<double> {
-  double d[2][8][kPad];             // P^-1 staging tiles, FP64 SpMV scratch
-  SpmvStage<double> s64[kWarps];    // staged SpMV rings (passes B, D), one per warp
+struct Smem {
+  SpmvStage<T> stage[kWarps];
+  double wred[kWarps][6];
+  double gres[6];
+  int flag;
+  // the CTAs solving one problem together: this CTA's rank among them and
+  // their number (the whole grid for a single solve, a group in a batch)
+  int team_rank, team_size;
+  int slot;           // batch: the problem the team works on
 };
-template <>
-union TileSmem<float> {
-  double d[2][8][kPad];             // FP64 SpMV scratch (true residual)
-  float f[2][16][kPad];             // P^-1 staging tiles
-  SpmvStage<float> s32[kWarps];     // staged SpMV rings (passes B, D), one per warp
-};
+
+template <class T>
+__device__ __forceinline__ SpmvStage<T>& spmv_stage(Smem<T>& sm) { return sm.stage[threadIdx.x >> 5]; }
+
+// The warp's scratch of kBLEN doubles (its ring is idle outside passes B and
+// D): the transposes of passes A and C, the block row of the FP64 SpMV.
+template <class T>
+__device__ __forceinline__ T* warp_scratch(Smem<T>& sm) { return spmv_stage(sm).z[0]; }
+template <class T>
+__device__ __forceinline__ double* spmv_row(Smem<T>& sm) { return reinterpret_cast<double*>(spmv_stage(sm).z[0]); }
 
 // P^-1 operand: FP64 rows, or the TF32 split of the FP32 P^-1 (hi, lo),
 // in rows of 64 values with the columns XOR-swizzled by the row (see the
@@ -115,29 +120,6 @@ struct PinvSmem<float> {
   uint32_t hi[kBLEN][kBLEN];
   uint32_t lo[kBLEN][kBLEN];
 };
-
-template <class T>
-struct Smem {
-  PinvSmem<T> P;
-  TileSmem<T> tile;
-  double wred[kWarps][6];
-  double gres[6];
-  int flag;
-  // the CTAs solving one problem together: this CTA's rank among them and
-  // their number (the whole grid for a single solve, a group in a batch)
-  int team_rank, team_size;
-  int slot;           // batch: the problem the team works on
-};
-
-// the warp's ring of the staged SpMV
-__device__ __forceinline__ SpmvStage<float>& spmv_stage(Smem<float>& sm) { return sm.tile.s32[threadIdx.x >> 5]; }
-__device__ __forceinline__ SpmvStage<double>& spmv_stage(Smem<double>& sm) { return sm.tile.s64[threadIdx.x >> 5]; }
-
-// the warp's block row of the FP64 staging tile, as SpMV scratch
-template <class SM>
-__device__ __forceinline__ double* spmv_row(SM& sm) {
-  return sm.tile.d[0][threadIdx.x >> 5];
-}
 
 // max that propagates NaN (fmax drops it, which would let a blown-up
 // residual read as converged)
@@ -213,8 +195,6 @@ struct Pinv<double> {
     }
     P = s.v;
   }
-  template <class SM>
-  __device__ __forceinline__ static double (*rows(SM& sm, int buf))[kPad] { return sm.tile.d[buf]; }
   __device__ __forceinline__ void apply(const double (*tile)[kPad], int w, int lane, int tb, int nvalid,
                                         double* __restrict__ z) const {
     const int g = lane >> 2, t = lane & 3;
@@ -232,20 +212,6 @@ struct Pinv<double> {
     if (2 * t + 1 < nvalid) z[(tb + 2 * t + 1) * kBLEN + 8 * w + g] = c1;
   }
 };
-
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // FP32: tiles of 16 blocks; warp w computes rows 16*(w&3).. of blocks
 // 8*(w>>2).. with m16n8k8 TF32 MMA.  Operands are split x = hi + lo (both
@@ -272,8 +238,6 @@ struct Pinv<float> {
     Ph = s.hi;
     Pl = s.lo;
   }
-  template <class SM>
-  __device__ __forceinline__ static float (*rows(SM& sm, int buf))[kPad] { return sm.tile.f[buf]; }
   __device__ __forceinline__ void apply(const float (*tile)[kPad], int w, int lane, int tb, int nvalid,
                                         float* __restrict__ z) const {
     const int g = lane >> 2, t = lane & 3, m = w & 3, nt = w >> 2;
@@ -494,17 +458,18 @@ struct MixedCtx {  // what the reliable update needs
 // replacement; MC the mean constraint (FP64 only).  Returns false if a
 // barrier gave up.
 template <class T, bool RU, bool MC>
-__device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const Pinv<T>& pin, const Problem<T>& V,
+__device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& pin, const Problem<T>& V,
                               double* __restrict__ red, int b0, int b1, int r0, int r1, const SolveParams& sp,
                               const MixedCtx& mx, IterState& st) {
   static_assert(!(MC && RU), "the mean constraint runs in the FP64 form only");
   using X = double;
   const MeshView& M = V.M;
-  constexpr int TB = Pinv<T>::kTile;
   constexpr int LV = Lane<T>::V, CB = Lane<T>::CB;  // 16-byte lane layout
-  static_assert(TB == CB * kWarps, "one chunk of each tile per warp");
+  constexpr int FN = Frag<T>::N;                    // values per lane in the fragment layout of passes A and C
+  static_assert(CB == Frag<T>::CB, "the layouts share the chunk");
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const Lane<T> L(lane);
+  T* const scratch = warp_scratch(sm);
   const double eps = 1e-21;
   // MC: the CTA whose SpMV computes the mean row records that row's own
   // product (its partials subtract it and add the sum h^2 v in its place)
@@ -532,44 +497,31 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const Pinv<T>& pin, c
       beta = (rho / (rho_prev + eps)) * (alpha / (omega + eps));
     }
     const T tb_beta = (T)beta, tb_omega = (T)omega;
-    // pass A: p = r + beta (p - omega nu); z = P^-1 p.  Warp w stages chunk w
-    // of each tile and loads its operands of the next tile before the
-    // tensor-core apply of the current one, so the loads overlap the apply.
+    // pass A: p = r + beta (p - omega nu); z = P^-1 p, warp by warp: the
+    // next chunk's operands are loaded before this chunk's block solve, so
+    // that the loads overlap it.
     {
-      T rr[LV], pp[LV], nn[LV];
-      auto load = [&](int tb) {
-        const int blk = tb + w * CB + L.bl;
-        if (blk < b1) {
-          const int i0 = blk * kBLEN + L.cell0;
-          ldv<LV>(V.r + i0, rr);
-          if (!zero_pnu) {
-            ldv<LV>(V.p + i0, pp);
-            ldv<LV>(V.nu + i0, nn);
-          }
+      T rr[FN], pp[FN], nn[FN];
+      auto load = [&](int blk) {
+        const int nv = b1 - blk;
+        ld_frag<T>(V.r, blk, nv, lane, rr);
+        if (!zero_pnu) {
+          ld_frag<T>(V.p, blk, nv, lane, pp);
+          ld_frag<T>(V.nu, blk, nv, lane, nn);
         }
       };
-      int buf = 0;
-      if (b0 < b1) load(b0);
-      for (int tb = b0; tb < b1; tb += TB) {
-        const int nvalid = (int)imin64(TB, b1 - tb);
-        auto tile = Pinv<T>::rows(sm, buf);
-        const int j = w * CB + L.bl;
-        T pv[LV];
-        if (j < nvalid) {
-          const int i0 = (tb + j) * kBLEN + L.cell0;
+      int blk = b0 + w * CB;
+      if (blk < b1) load(blk);
+      for (; blk < b1; blk += kWarps * CB) {
+        const int nv = b1 - blk;
+        T pv[FN];
 #pragma unroll
-          for (int k = 0; k < LV; ++k) pv[k] = zero_pnu ? rr[k] : rr[k] + tb_beta * (pp[k] - tb_omega * nn[k]);
-          if (restart_now) stv<LV>(V.rh + i0, rr);
-          stv<LV>(V.p + i0, pv);
-        } else {
-#pragma unroll
-          for (int k = 0; k < LV; ++k) pv[k] = T(0);
-        }
-        stv<LV>(&tile[j][L.cell0], pv);
-        if (tb + TB < b1) load(tb + TB);
-        __syncthreads();
-        pin.apply(tile, w, lane, tb, nvalid, V.z);
-        buf ^= 1;
+        for (int k = 0; k < FN; ++k) pv[k] = zero_pnu ? rr[k] : rr[k] + tb_beta * (pp[k] - tb_omega * nn[k]);
+        if (restart_now) st_frag<T>(V.rh, blk, nv, lane, rr);
+        st_frag<T>(V.p, blk, nv, lane, pv);
+        if (blk + kWarps * CB < b1) load(blk + kWarps * CB);
+        pin.apply(pv, scratch, lane);
+        st_frag<T>(V.z, blk, nv, lane, pv);
       }
       zero_pnu = false;
     }
@@ -609,36 +561,22 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const Pinv<T>& pin, c
     const T ta = (T)alpha;
     // pass C: s = r - alpha nu (in place of r); z2 = P^-1 s
     {
-      T rr[LV], nn[LV];
-      auto load = [&](int tb) {
-        const int blk = tb + w * CB + L.bl;
-        if (blk < b1) {
-          const int i0 = blk * kBLEN + L.cell0;
-          ldv<LV>(V.r + i0, rr);
-          ldv<LV>(V.nu + i0, nn);
-        }
+      T rr[FN], nn[FN];
+      auto load = [&](int blk) {
+        ld_frag<T>(V.r, blk, b1 - blk, lane, rr);
+        ld_frag<T>(V.nu, blk, b1 - blk, lane, nn);
       };
-      int buf = 0;
-      if (b0 < b1) load(b0);
-      for (int tb = b0; tb < b1; tb += TB) {
-        const int nvalid = (int)imin64(TB, b1 - tb);
-        auto tile = Pinv<T>::rows(sm, buf);
-        const int j = w * CB + L.bl;
-        T sv[LV];
-        if (j < nvalid) {
-          const int i0 = (tb + j) * kBLEN + L.cell0;
+      int blk = b0 + w * CB;
+      if (blk < b1) load(blk);
+      for (; blk < b1; blk += kWarps * CB) {
+        const int nv = b1 - blk;
+        T sv[FN];
 #pragma unroll
-          for (int k = 0; k < LV; ++k) sv[k] = rr[k] - ta * nn[k];
-          stv<LV>(V.r + i0, sv);
-        } else {
-#pragma unroll
-          for (int k = 0; k < LV; ++k) sv[k] = T(0);
-        }
-        stv<LV>(&tile[j][L.cell0], sv);
-        if (tb + TB < b1) load(tb + TB);
-        __syncthreads();
-        pin.apply(tile, w, lane, tb, nvalid, V.z2);
-        buf ^= 1;
+        for (int k = 0; k < FN; ++k) sv[k] = rr[k] - ta * nn[k];
+        st_frag<T>(V.r, blk, nv, lane, sv);
+        if (blk + kWarps * CB < b1) load(blk + kWarps * CB);
+        pin.apply(sv, scratch, lane);
+        st_frag<T>(V.z2, blk, nv, lane, sv);
       }
     }
     if (!B.sync(&sm.flag, 3)) return false;
@@ -847,7 +785,7 @@ __device__ __forceinline__ void write_stats(const SM& sm, DevStats* stats, const
 // [b0,b1) is this CTA's block range, [r0,r1) its explicit rows.
 // MC: the mean constraint (sp.mean_row).
 template <bool MC>
-__device__ bool solve_fp64(Smem<double>& sm, GridBarrier& B, const Pinv<double>& pin, const Problem64& pr,
+__device__ bool solve_fp64(Smem<double>& sm, GridBarrier& B, const SineSolve<double>& pin, const Problem64& pr,
                            const SolveParams& sp, double* __restrict__ red, int b0, int b1, int r0,
                            int r1) {
   const MeshView& M = pr.M;
@@ -931,7 +869,7 @@ __device__ bool solve_fp64(Smem<double>& sm, GridBarrier& B, const Pinv<double>&
 }
 
 // Mixed-precision solve of one problem by the team.
-__device__ bool solve_mixed(Smem<float>& sm, GridBarrier& B, const Pinv<float>& pin, const ProblemMixed& pr,
+__device__ bool solve_mixed(Smem<float>& sm, GridBarrier& B, const SineSolve<float>& pin, const ProblemMixed& pr,
                             const SolveParams& sp, double* __restrict__ red, int b0, int b1, int r0,
                             int r1) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1007,8 +945,8 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab64(c
     sm.team_rank = blockIdx.x;
     sm.team_size = gridDim.x;
   }
-  Pinv<double> pin;
-  pin.load(sm.P, S.P, nullptr);
+  SineSolve<double> pin;
+  pin.init();
   __syncthreads();
   solve_fp64<false>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
 }
@@ -1025,8 +963,8 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm)
     sm.team_rank = blockIdx.x;
     sm.team_size = gridDim.x;
   }
-  Pinv<double> pin;
-  pin.load(sm.P, S.P, nullptr);
+  SineSolve<double> pin;
+  pin.init();
   __syncthreads();
   solve_fp64<true>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
 }
@@ -1040,8 +978,8 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab_mix
     sm.team_rank = blockIdx.x;
     sm.team_size = gridDim.x;
   }
-  Pinv<float> pin;
-  pin.load(sm.P, nullptr, S.P32);
+  SineSolve<float> pin;
+  pin.init();
   __syncthreads();
   solve_mixed(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
 }
@@ -1059,8 +997,8 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
     sm.team_rank = blockIdx.x;
     sm.team_size = gridDim.x;
   }
-  Pinv<double> pin;
-  pin.load(sm.P, S.P, nullptr);
+  SineSolve<double> pin;
+  pin.init();
   __syncthreads();
   solve_fp64<false>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
 }
@@ -1075,8 +1013,8 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
     sm.team_rank = blockIdx.x;
     sm.team_size = gridDim.x;
   }
-  Pinv<float> pin;
-  pin.load(sm.P, nullptr, S.P32);
+  SineSolve<float> pin;
+  pin.init();
   __syncthreads();
   solve_mixed(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
 }
@@ -1102,8 +1040,8 @@ __device__ __forceinline__ void batch_body(const BatchArgs& A) {
     sm.team_rank = rank;
     sm.team_size = team;
   }
-  typename std::conditional<MIXED, Pinv<float>, Pinv<double>>::type pin;
-  pin.load(sm.P, A.P, A.P32);
+  SineSolve<KT> pin;
+  pin.init();
   __syncthreads();
   double* red = A.red + (size_t)g * kRedQ * team;
   while (true) {

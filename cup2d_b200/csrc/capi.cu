@@ -646,7 +646,6 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     SolveArgsMixed a{};
     a.prob = ProblemMixed{h->mesh.view(), d_b, d_x, h->xo.p, h->f_r.p, h->f_rh.p, h->f_p.p, h->f_nu.p,
                           h->f_t.p, h->f_z.p, h->f_z2.p, h->dstats.p};
-    a.P32 = h->P32;
     a.red = h->red.p;
     a.bar = h->bar.p;
     a.abort_flag = h->abort_flag.p;
@@ -660,7 +659,6 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     SolveArgs64 a{};
     a.prob = Problem64{h->mesh.view(), d_b, d_x, h->xo.p, h->r.p, h->rh.p, h->p.p, h->nu.p, h->t.p, h->z.p,
                        h->z2.p, h->dstats.p};
-    a.P = h->P;
     a.red = h->red.p;
     a.bar = h->bar.p;
     a.abort_flag = h->abort_flag.p;
@@ -1026,8 +1024,6 @@ struct cup2d_batch {
   DevBuf<unsigned> bars;
   DevBuf<int> slots, queue, abort_flag;
   DevBuf<DevStats> dstats;
-  const double* P = nullptr;  // the device's shared P^-1
-  const float* P32 = nullptr;
   std::vector<Problem64> h_p64;
   std::vector<ProblemMixed> h_pmx;
   std::vector<DevStats> hstats;
@@ -1123,8 +1119,7 @@ int cup2d_batch_create(int32_t n, const cup2d_forest* forests, const cup2d_solve
   const int gmax = std::max(B->grid64, B->gridmx);
   if ((st = B->d_p64.ensure(n)) || (st = B->d_pmx.ensure(n)) || (st = B->d_order.ensure(n)) ||
       (st = B->red.ensure((int64_t)kRedQ * gmax)) || (st = B->bars.ensure(gmax)) || (st = B->slots.ensure(gmax)) ||
-      (st = B->queue.ensure(1)) || (st = B->abort_flag.ensure(1)) || (st = B->dstats.ensure(n)) ||
-      (st = shared_pinv(&B->P, &B->P32))) {
+      (st = B->queue.ensure(1)) || (st = B->abort_flag.ensure(1)) || (st = B->dstats.ensure(n))) {
     cup2d_batch_destroy(B);
     return st;
   }
@@ -1215,8 +1210,6 @@ int batch_prepare(cup2d_batch* B, const double* const* d_b, double* const* d_x, 
   a.order = B->d_order.p;
   a.nprob = n;
   a.team = team;
-  a.P = B->P;
-  a.P32 = B->P32;
   a.red = B->red.p;
   a.bars = B->bars.p;
   a.slots = B->slots.p;
@@ -1590,7 +1583,6 @@ int handle_view(const cup2d_poisson* h, HandleView* out) {
   if (!h || !out || h->nb <= 0) return CUP2D_INVALID_ARGUMENT;
   out->device = h->device;
   out->M = h->mesh.view();
-  out->P = h->P;
   out->nb = h->nb;
   out->grid = h->grid_for(h->grid64);
   out->opts = h->opts;

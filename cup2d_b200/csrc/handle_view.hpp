@@ -13,7 +13,6 @@ namespace cup2d {
 struct HandleView {
   int device;                              // the handle's CUDA device
   MeshView M;                              // assembled operator (device)
-  const double* P;                         // FP64 P^-1 (device)
   int64_t nb;                              // blocks
   int grid;                                // CTAs the FP64 solve would use
   cup2d_solve_opts opts;

@@ -125,7 +125,6 @@ struct SolveParams {
 // and refer to the problem and parameters in place (no per-thread copies).
 struct SolveArgs64 {
   Problem64 prob;       // operator, b, x (x0 in, solution out), Krylov vectors
-  const double* P;      // 64x64 row-major P^-1
   double* red;          // [kRedQ][grid]
   unsigned* bar;        // arrival counter, zeroed before launch
   int* abort_flag;      // zeroed before launch
@@ -137,7 +136,6 @@ struct SolveArgs64 {
 // Mixed precision: FP32 Krylov vectors, FP64 solution and true residual.
 struct SolveArgsMixed {
   ProblemMixed prob;
-  const float* P32;     // 64x64 row-major FP32 P^-1 (rounded from the FP64 build)
   double* red;
   unsigned* bar;
   int* abort_flag;
@@ -154,8 +152,6 @@ struct BatchArgs {
   const int32_t* order;     // [nprob] queue order
   int nprob;
   int team;                 // CTAs per problem; the grid is a multiple of it
-  const double* P;          // FP64 P^-1
-  const float* P32;         // FP32 P^-1
   double* red;              // [groups][kRedQ][team]
   unsigned* bars;           // [groups] barrier counters, zeroed
   int* slots;               // [groups]

@@ -136,7 +136,6 @@ extern "C" int cup2d_poisson_solve_device_noalloc(cup2d_poisson* h, const double
                      vec + 6 * stride,  // z
                      vec + 7 * stride,  // z2
                      reinterpret_cast<DevStats*>(base + kOffStats)};
-  a.P = v.P;
   a.red = reinterpret_cast<double*>(base + kOffRed);
   a.bar = reinterpret_cast<unsigned*>(base + kOffBar);
   a.abort_flag = reinterpret_cast<int*>(base + kOffAbort);
