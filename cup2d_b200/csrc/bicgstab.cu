@@ -60,25 +60,8 @@ namespace cup2d {
 
 namespace {
 
-constexpr int kWarps = kSolveThreads / 32;
 constexpr int kPad = 68;  // staged block row (conflict-free fragment loads)
 constexpr int kMaxSweep = 64;  // mixed: longest FP32 sweep between true residuals
-
-enum : int {
-  Q_INIT = 0,   // 3: |A x0|_inf, |r0|_inf, |r0|^2
-  Q_RHNU = 3,   // pass B
-  Q_TS = 4,     // pass D: (t,s), (t,t)
-  Q_RMAX = 6,   // pass E: |r|_inf, (rhat,r), |r|^2, |rhat|^2
-  Q_HX = 10,    // mean removal: sum h^2 x, sum h^2
-  Q_RU = 12,    // true residual: |r64|_inf, (rhat,r), |r|^2, |rhat|^2, |r32|_inf
-  Q_SUMB = 17,  // sum b
-  // single solves with the mean constraint (kRedQMean slots)
-  Q_MB = 20,    // pass B: (rhat,nu), sum h^2 z, rhat_m nu_m, rhat_m
-  Q_MD = 24,    // pass D: (t,s), (t,t), sum h^2 z2, t_m s_m, t_m t_m, s_m
-  Q_MX = 30     // sum h^2 x0
-};
-static_assert(Q_SUMB + 1 <= kRedQ, "reduction slots");
-static_assert(Q_MX + 1 <= kRedQMean, "reduction slots (mean constraint)");
 
 // Shared memory of the solve kernels, per precision T of the Krylov vectors:
 // per warp one ring of the staged SpMV, which also serves as the scratch of
@@ -87,13 +70,8 @@ static_assert(Q_MX + 1 <= kRedQMean, "reduction slots (mean constraint)");
 template <class T>
 struct Smem {
   SpmvStage<T> stage[kWarps];
-  double wred[kWarps][6];
-  double gres[6];
-  int flag;
-  // the CTAs solving one problem together: this CTA's rank among them and
-  // their number (the whole grid for a single solve, a group in a batch)
-  int team_rank, team_size;
-  int slot;           // batch: the problem the team works on
+  Team team;
+  int slot;  // batch: the problem the team works on
 };
 
 template <class T>
@@ -120,57 +98,6 @@ struct PinvSmem<float> {
   uint32_t hi[kBLEN][kBLEN];
   uint32_t lo[kBLEN][kBLEN];
 };
-
-// max that propagates NaN (fmax drops it, which would let a blown-up
-// residual read as converged)
-__device__ __forceinline__ double nanmax(double a, double b) { return (a > b || a != a) ? a : b; }
-
-template <int NV, class SM>
-__device__ __forceinline__ void cta_partials(SM& sm, const double (&v)[NV], unsigned is_max,
-                                             double* __restrict__ red, int q0) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double r = v[q];
-    if ((is_max >> q) & 1u) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) r = nanmax(r, __shfl_xor_sync(kFull, r, o));
-    } else {
-      r = warp_sum(r);
-    }
-    if (lane == 0) sm.wred[w][q] = r;
-  }
-  __syncthreads();
-  if (threadIdx.x < NV) {
-    const int q = threadIdx.x;
-    double acc = sm.wred[0][q];
-    for (int k = 1; k < kWarps; ++k)
-      acc = ((is_max >> q) & 1u) ? nanmax(acc, sm.wred[k][q]) : acc + sm.wred[k][q];
-    red[(q0 + q) * sm.team_size + sm.team_rank] = acc;
-  }
-}
-
-template <int NV, class SM>
-__device__ __forceinline__ void grid_reduce(SM& sm, unsigned is_max, const double* __restrict__ red, int q0) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (w < NV) {
-    const bool mx = (is_max >> w) & 1u;
-    const double* src = red + (q0 + w) * sm.team_size;
-    double acc = 0.0;
-    for (int j = lane; j < sm.team_size; j += 32) {
-      const double v = __ldcg(src + j);
-      acc = mx ? nanmax(acc, v) : acc + v;
-    }
-    if (mx) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc = nanmax(acc, __shfl_xor_sync(kFull, acc, o));
-    } else {
-      acc = warp_sum(acc);
-    }
-    if (lane == 0) sm.gres[w] = acc;
-  }
-  __syncthreads();
-}
 
 // ------------------------------------------------ P^-1 tile application ----
 
@@ -386,12 +313,13 @@ struct EpiTS {
 };
 
 // Mixed form: r = (b - mean_b) - A x in FP64, stored as FP32 (and as rhat
-// when set_rh); partials |r64|_inf, (rhat,r), |r|^2, |rhat|^2, |r32|_inf.
+// when set_rh); B.out: |r64|_inf, (rhat,r), |r|^2, |rhat|^2, |r32|_inf over the
+// team.  x must be visible to the team.  Returns false if the wait gave up.
 template <class SM>
-__device__ __forceinline__ void true_residual(SM& sm, const MeshView& M, const double* __restrict__ b,
+__device__ __forceinline__ bool true_residual(SM& sm, Team& B, const MeshView& M, const double* __restrict__ b,
                                               double mean_b, const double* __restrict__ x, float* __restrict__ r,
-                                              float* __restrict__ rh, bool set_rh, double* __restrict__ red,
-                                              int b0, int b1, int r0, int r1) {
+                                              float* __restrict__ rh, bool set_rh, int b0, int b1, int r0, int r1,
+                                              int phase) {
   struct Epi {
     const double* b;
     double mean_b;
@@ -441,7 +369,7 @@ __device__ __forceinline__ void true_residual(SM& sm, const MeshView& M, const d
     }
   } epi{b, mean_b, r, rh, set_rh, {0.0, 0.0, 0.0, 0.0, 0.0}};
   spmv_range<double>(M, x, b0, b1, r0, r1, epi, spmv_row(sm));
-  cta_partials<5>(sm, epi.v, 0x11u, red, Q_RU);
+  return B.reduce<5>(epi.v, 0x11u, phase);
 }
 
 struct MixedCtx {  // what the reliable update needs
@@ -458,8 +386,8 @@ struct MixedCtx {  // what the reliable update needs
 // replacement; MC the mean constraint (FP64 only).  Returns false if a
 // barrier gave up.
 template <class T, bool RU, bool MC>
-__device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& pin, const Problem<T>& V,
-                              double* __restrict__ red, int b0, int b1, int r0, int r1, const SolveParams& sp,
+__device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, const Problem<T>& V,
+                              int b0, int b1, int r0, int r1, const SolveParams& sp,
                               const MixedCtx& mx, IterState& st) {
   static_assert(!(MC && RU), "the mean constraint runs in the FP64 form only");
   using X = double;
@@ -525,8 +453,9 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
       }
       zero_pnu = false;
     }
-    if (!B.sync(&sm.flag, 1)) return false;
+    if (!B.sync(1)) return false;
     // pass B: nu = A z; (rhat, nu)
+    double rhnu;
     {
       EpiRhNu<T> epi{V.rh, V.nu, 0.0};
       spmv_range_staged<T>(M, V.z, V.rh, b0, b1, r0, r1, epi, spmv_stage(sm));
@@ -539,23 +468,17 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
           v[2] = dprod(rv, y);
           v[3] = (double)rv;
         }
-        cta_partials<4>(sm, v, 0u, red, Q_MB);
+        if (!B.reduce<4>(v, 0u, 2)) return false;
+        const double* const o = B.out;
+        const T m = (T)o[1];
+        rhnu = (o[0] - o[2]) + o[3] * (double)m;
+        if (threadIdx.x == 0 && owns_row(sp.mean_row, b0, b1)) V.nu[sp.mean_row] = m;
+        __syncthreads();
       } else {
         const double v[1] = {epi.acc};
-        cta_partials<1>(sm, v, 0u, red, Q_RHNU);
+        if (!B.reduce<1>(v, 0u, 2)) return false;
+        rhnu = B.out[0];
       }
-    }
-    if (!B.sync(&sm.flag, 2)) return false;
-    double rhnu;
-    if constexpr (MC) {
-      grid_reduce<4>(sm, 0u, red, Q_MB);
-      const T m = (T)sm.gres[1];
-      rhnu = (sm.gres[0] - sm.gres[2]) + sm.gres[3] * (double)m;
-      if (threadIdx.x == 0 && owns_row(sp.mean_row, b0, b1)) V.nu[sp.mean_row] = m;
-      __syncthreads();
-    } else {
-      grid_reduce<1>(sm, 0u, red, Q_RHNU);
-      rhnu = sm.gres[0];
     }
     alpha = rho / (rhnu + eps);
     const T ta = (T)alpha;
@@ -579,7 +502,7 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
         st_frag<T>(V.z2, blk, nv, lane, sv);
       }
     }
-    if (!B.sync(&sm.flag, 3)) return false;
+    if (!B.sync(3)) return false;
     // pass D: t = A z2; (t,s), (t,t)
     {
       EpiTS<T> epi{V.r, V.t, 0.0, 0.0};
@@ -593,24 +516,19 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
           v[4] = dprod(y, y);
           v[5] = (double)sv;
         }
-        cta_partials<6>(sm, v, 0u, red, Q_MD);
+        if (!B.reduce<6>(v, 0u, 4)) return false;
+        const double* const o = B.out;
+        const T m = (T)o[2];
+        const double ts = (o[0] - o[3]) + o[5] * (double)m;
+        const double tt = (o[1] - o[4]) + dprod(m, m);
+        omega = ts / (tt + eps);
+        if (threadIdx.x == 0 && owns_row(sp.mean_row, b0, b1)) V.t[sp.mean_row] = m;
+        __syncthreads();
       } else {
         const double v[2] = {epi.ts, epi.tt};
-        cta_partials<2>(sm, v, 0u, red, Q_TS);
+        if (!B.reduce<2>(v, 0u, 4)) return false;
+        omega = B.out[0] / (B.out[1] + eps);
       }
-    }
-    if (!B.sync(&sm.flag, 4)) return false;
-    if constexpr (MC) {
-      grid_reduce<6>(sm, 0u, red, Q_MD);
-      const T m = (T)sm.gres[2];
-      const double ts = (sm.gres[0] - sm.gres[3]) + sm.gres[5] * (double)m;
-      const double tt = (sm.gres[1] - sm.gres[4]) + dprod(m, m);
-      omega = ts / (tt + eps);
-      if (threadIdx.x == 0 && owns_row(sp.mean_row, b0, b1)) V.t[sp.mean_row] = m;
-      __syncthreads();
-    } else {
-      grid_reduce<2>(sm, 0u, red, Q_TS);
-      omega = sm.gres[0] / (sm.gres[1] + eps);
     }
     const T to = (T)omega;
     // pass E: x += alpha z, then x += omega z2 (the reference's two axpys,
@@ -650,14 +568,12 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
         stv<LV>(V.x + i0, xn);
         stv<LV>(V.r + i0, rn);
       }
-      cta_partials<4>(sm, v, 0x1u, red, Q_RMAX);
+      if (!B.reduce<4>(v, 0x1u, 5)) return false;
     }
-    if (!B.sync(&sm.flag, 5)) return false;
-    grid_reduce<4>(sm, 0x1u, red, Q_RMAX);
-    double error = sm.gres[0];
-    double rho_new = sm.gres[1];
-    nr = sm.gres[2];
-    nrh = sm.gres[3];
+    double error = B.out[0];
+    double rho_new = B.out[1];
+    nr = B.out[2];
+    nrh = B.out[3];
     if (!(error == error) || !(rho_new == rho_new)) {  // non-finite: stop, keep the best iterate
       st.best_is_x = false;
       ++k;
@@ -673,16 +589,14 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
       if (claims || sqrt(nr) < mx.delta * rmax_since || since >= kMaxSweep) {
         since = 0;
         // pass E's barrier already ordered every CTA's x update before this
-        true_residual(sm, M, mx.b, mx.mean_b, V.x, V.r, V.rh, mx.restart, red, b0, b1, r0, r1);
-        if (!B.sync(&sm.flag, 6)) return false;
-        grid_reduce<5>(sm, 0x11u, red, Q_RU);
+        if (!true_residual(sm, B, M, mx.b, mx.mean_b, V.x, V.r, V.rh, mx.restart, b0, b1, r0, r1, 6)) return false;
         ++st.updates;
         refreshed = true;
-        st.err_true = sm.gres[0];
-        rho_new = sm.gres[1];
-        nr = sm.gres[2];
-        nrh = sm.gres[3];
-        error = sm.gres[4];
+        st.err_true = B.out[0];
+        rho_new = B.out[1];
+        nr = B.out[2];
+        nrh = B.out[3];
+        error = B.out[4];
         rmax_since = sqrt(nr);
         if ((st.err_true <= mx.tol_abs) || (st.err_true / st.err_init <= mx.tol_rel)) {
           st.err_opt = fmin(st.err_opt, st.err_true);
@@ -730,8 +644,8 @@ __device__ bool bicgstab_loop(Smem<T>& sm, GridBarrier& B, const SineSolve<T>& p
 // x -= sum(h^2 x)/sum(h^2) over the CTA's blocks (ExpAMRSolver.cpp:383-415);
 // x already holds the final iterate.
 template <class SM>
-__device__ bool subtract_mean(SM& sm, GridBarrier& B, const MeshView& M, double* __restrict__ x,
-                              double* __restrict__ red, int b0, int b1) {
+__device__ bool subtract_mean(SM& sm, Team& B, const MeshView& M, double* __restrict__ x,
+                              int b0, int b1) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double v[2] = {0.0, 0.0};
   for (int blk = b0 + w; blk < b1; blk += kWarps) {
@@ -740,10 +654,8 @@ __device__ bool subtract_mean(SM& sm, GridBarrier& B, const MeshView& M, double*
     v[0] += (__ldcg(x + o + lane) + __ldcg(x + o + lane + 32)) * (hb * hb);
     v[1] += 2.0 * (hb * hb);
   }
-  cta_partials<2>(sm, v, 0u, red, Q_HX);
-  if (!B.sync(&sm.flag, 7)) return false;
-  grid_reduce<2>(sm, 0u, red, Q_HX);
-  const double avg = sm.gres[0] / sm.gres[1];
+  if (!B.reduce<2>(v, 0u, 7)) return false;
+  const double avg = B.out[0] / B.out[1];
   for (int blk = b0 + w; blk < b1; blk += kWarps) {
     const int o = blk * kBLEN;
     x[o + lane] = __ldcg(x + o + lane) - avg;
@@ -766,10 +678,9 @@ __device__ __forceinline__ void take_best(bool best_is_x, double* __restrict__ x
 
 // ============================================ one problem, one team ========
 
-template <class SM>
-__device__ __forceinline__ void write_stats(const SM& sm, DevStats* stats, const IterState& st, int refinements,
+__device__ __forceinline__ void write_stats(const Team& B, DevStats* stats, const IterState& st, int refinements,
                                             double err_final, double norm_ax0) {
-  if (sm.team_rank == 0 && threadIdx.x == 0) {
+  if (B.rank == 0 && threadIdx.x == 0) {
     stats->status = st.status;
     stats->iterations = st.iters;
     stats->restarts = st.restarts;
@@ -785,17 +696,15 @@ __device__ __forceinline__ void write_stats(const SM& sm, DevStats* stats, const
 // [b0,b1) is this CTA's block range, [r0,r1) its explicit rows.
 // MC: the mean constraint (sp.mean_row).
 template <bool MC>
-__device__ bool solve_fp64(Smem<double>& sm, GridBarrier& B, const SineSolve<double>& pin, const Problem64& pr,
-                           const SolveParams& sp, double* __restrict__ red, int b0, int b1, int r0,
+__device__ bool solve_fp64(Smem<double>& sm, Team& B, const SineSolve<double>& pin, const Problem64& pr,
+                           const SolveParams& sp, int b0, int b1, int r0,
                            int r1) {
   const MeshView& M = pr.M;
   double x0sum = 0.0;  // MC: sum h^2 x0, the mean row of A x0
   if constexpr (MC) {
     const double v[1] = {hsum_part(M, pr.x, b0, b1)};
-    cta_partials<1>(sm, v, 0u, red, Q_MX);
-    if (!B.sync(&sm.flag, 9)) return false;
-    grid_reduce<1>(sm, 0u, red, Q_MX);
-    x0sum = sm.gres[0];
+    if (!B.reduce<1>(v, 0u, 9)) return false;
+    x0sum = B.out[0];
   }
   // r = b - A x0, rhat = r, |A x0|_inf, |r0|_inf (BiCGSTAB.cu:430-465)
   {
@@ -844,33 +753,31 @@ __device__ bool solve_fp64(Smem<double>& sm, GridBarrier& B, const SineSolve<dou
       }
     } epi{pr.b, pr.r, pr.rh, sp.mean_row, x0sum, {0.0, 0.0, 0.0}};
     spmv_range<double>(M, pr.x, b0, b1, r0, r1, epi, spmv_row(sm));
-    cta_partials<3>(sm, epi.v, 0x3u, red, Q_INIT);
+    if (!B.reduce<3>(epi.v, 0x3u, 0)) return false;
   }
-  if (!B.sync(&sm.flag, 0)) return false;
-  grid_reduce<3>(sm, 0x3u, red, Q_INIT);
   IterState st;
-  const double norm_ax0 = sm.gres[0];
-  st.err_init = sm.gres[1];
+  const double norm_ax0 = B.out[0];
+  st.err_init = B.out[1];
   st.err_opt = st.err_init;
   st.err_true = st.err_init;
-  st.rho = st.nr = st.nrh = sm.gres[2];
+  st.rho = st.nr = st.nrh = B.out[2];
   st.restarts = 0;
   st.iters = 0;
   st.updates = 0;
   st.best_is_x = true;
   st.status = CUP2D_NOT_CONVERGED;
   const MixedCtx none{};
-  if (!bicgstab_loop<double, false, MC>(sm, B, pin, pr, red, b0, b1, r0, r1, sp, none, st))
+  if (!bicgstab_loop<double, false, MC>(sm, B, pin, pr, b0, b1, r0, r1, sp, none, st))
     return false;
   take_best(st.best_is_x, pr.x, pr.xo, b0, b1);
-  if (sp.subtract_mean && !subtract_mean(sm, B, M, pr.x, red, b0, b1)) return false;
-  write_stats(sm, pr.stats, st, 0, st.err_opt, norm_ax0);
+  if (sp.subtract_mean && !subtract_mean(sm, B, M, pr.x, b0, b1)) return false;
+  write_stats(B, pr.stats, st, 0, st.err_opt, norm_ax0);
   return true;
 }
 
 // Mixed-precision solve of one problem by the team.
-__device__ bool solve_mixed(Smem<float>& sm, GridBarrier& B, const SineSolve<float>& pin, const ProblemMixed& pr,
-                            const SolveParams& sp, double* __restrict__ red, int b0, int b1, int r0,
+__device__ bool solve_mixed(Smem<float>& sm, Team& B, const SineSolve<float>& pin, const ProblemMixed& pr,
+                            const SolveParams& sp, int b0, int b1, int r0,
                             int r1) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // Neumann compatibility: project b to zero sum (sum b / n)
@@ -880,27 +787,23 @@ __device__ bool solve_mixed(Smem<float>& sm, GridBarrier& B, const SineSolve<flo
       const int o = blk * kBLEN;
       v[0] += __ldg(pr.b + o + lane) + __ldg(pr.b + o + lane + 32);
     }
-    cta_partials<1>(sm, v, 0u, red, Q_SUMB);
+    if (!B.reduce<1>(v, 0u, 8)) return false;
   }
-  if (!B.sync(&sm.flag, 8)) return false;
-  grid_reduce<1>(sm, 0u, red, Q_SUMB);
   MixedCtx mx;
   mx.b = pr.b;
-  mx.mean_b = sm.gres[0] / (double)(pr.M.nb * kBLEN);
+  mx.mean_b = B.out[0] / (double)(pr.M.nb * kBLEN);
   mx.delta = sp.reliable_delta;
   mx.tol_abs = sp.tol_abs;
   mx.tol_rel = sp.tol_rel;
   mx.restart = sp.reliable_restart != 0;
-  true_residual(sm, pr.M, pr.b, mx.mean_b, pr.x, pr.r, pr.rh, true, red, b0, b1, r0, r1);
-  if (!B.sync(&sm.flag, 0)) return false;
-  grid_reduce<5>(sm, 0x11u, red, Q_RU);
+  if (!true_residual(sm, B, pr.M, pr.b, mx.mean_b, pr.x, pr.r, pr.rh, true, b0, b1, r0, r1, 0)) return false;
   IterState st;
-  st.err_init = sm.gres[0];
-  st.err_true = sm.gres[0];
-  st.err_opt = sm.gres[0];  // best true residual: x0's
-  st.rho = sm.gres[1];
-  st.nr = sm.gres[2];
-  st.nrh = sm.gres[3];
+  st.err_init = B.out[0];
+  st.err_true = B.out[0];
+  st.err_opt = B.out[0];  // best true residual: x0's
+  st.rho = B.out[1];
+  st.nr = B.out[2];
+  st.nrh = B.out[3];
   st.restarts = 0;
   st.iters = 0;
   st.updates = 0;
@@ -909,12 +812,12 @@ __device__ bool solve_mixed(Smem<float>& sm, GridBarrier& B, const SineSolve<flo
   const bool done0 = st.err_true <= sp.tol_abs || st.err_true == 0.0;
   if (done0) {
     st.status = CUP2D_OK;
-  } else if (!bicgstab_loop<float, true, false>(sm, B, pin, pr, red, b0, b1, r0, r1, sp, mx, st)) {
+  } else if (!bicgstab_loop<float, true, false>(sm, B, pin, pr, b0, b1, r0, r1, sp, mx, st)) {
     return false;
   }
   take_best(st.best_is_x, pr.x, pr.xo, b0, b1);
-  if (sp.subtract_mean && !subtract_mean(sm, B, pr.M, pr.x, red, b0, b1)) return false;
-  write_stats(sm, pr.stats, st, st.updates, st.status == CUP2D_OK ? st.err_true : st.err_opt, 0.0);
+  if (sp.subtract_mean && !subtract_mean(sm, B, pr.M, pr.x, b0, b1)) return false;
+  write_stats(B, pr.stats, st, st.updates, st.status == CUP2D_OK ? st.err_true : st.err_opt, 0.0);
   return true;
 }
 
@@ -940,15 +843,12 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab64(c
   Smem<double>& sm = solve_smem<double>();
   const int b0 = share(S.prob.M.nb, blockIdx.x, gridDim.x), b1 = share(S.prob.M.nb, blockIdx.x + 1, gridDim.x);
   const int r0 = share(S.prob.M.R, blockIdx.x, gridDim.x), r1 = share(S.prob.M.R, blockIdx.x + 1, gridDim.x);
-  GridBarrier B{S.bar, S.abort_flag, gridDim.x, globaltimer_ns() + S.timeout_ns, 0u, S.prof, globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = blockIdx.x;
-    sm.team_size = gridDim.x;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0) B.init(blockIdx.x, gridDim.x, S.bar, S.red, S.abort_flag, S.timeout_ns, S.prof);
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<false>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
+  solve_fp64<false>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
 }
 
 // With bMeanConstraint: the same solve on the system whose row S.sp.mean_row
@@ -958,30 +858,24 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm)
   Smem<double>& sm = solve_smem<double>();
   const int b0 = share(S.prob.M.nb, blockIdx.x, gridDim.x), b1 = share(S.prob.M.nb, blockIdx.x + 1, gridDim.x);
   const int r0 = share(S.prob.M.R, blockIdx.x, gridDim.x), r1 = share(S.prob.M.R, blockIdx.x + 1, gridDim.x);
-  GridBarrier B{S.bar, S.abort_flag, gridDim.x, globaltimer_ns() + S.timeout_ns, 0u, S.prof, globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = blockIdx.x;
-    sm.team_size = gridDim.x;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0) B.init(blockIdx.x, gridDim.x, S.bar, S.red, S.abort_flag, S.timeout_ns, S.prof);
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<true>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
+  solve_fp64<true>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab_mixed(const __grid_constant__ SolveArgsMixed S) {
   Smem<float>& sm = solve_smem<float>();
   const int b0 = share(S.prob.M.nb, blockIdx.x, gridDim.x), b1 = share(S.prob.M.nb, blockIdx.x + 1, gridDim.x);
   const int r0 = share(S.prob.M.R, blockIdx.x, gridDim.x), r1 = share(S.prob.M.R, blockIdx.x + 1, gridDim.x);
-  GridBarrier B{S.bar, S.abort_flag, gridDim.x, globaltimer_ns() + S.timeout_ns, 0u, S.prof, globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = blockIdx.x;
-    sm.team_size = gridDim.x;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0) B.init(blockIdx.x, gridDim.x, S.bar, S.red, S.abort_flag, S.timeout_ns, S.prof);
   SineSolve<float> pin;
   pin.init();
   __syncthreads();
-  solve_mixed(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
+  solve_mixed(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
 }
 
 
@@ -992,15 +886,12 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
   Smem<double>& sm = solve_smem<double>();
   const int b0 = share(S.prob.M.nb, blockIdx.x, gridDim.x), b1 = share(S.prob.M.nb, blockIdx.x + 1, gridDim.x);
   const int r0 = share(S.prob.M.R, blockIdx.x, gridDim.x), r1 = share(S.prob.M.R, blockIdx.x + 1, gridDim.x);
-  GridBarrier B{S.bar, S.abort_flag, gridDim.x, globaltimer_ns() + S.timeout_ns, 0u, S.prof, globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = blockIdx.x;
-    sm.team_size = gridDim.x;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0) B.init(blockIdx.x, gridDim.x, S.bar, S.red, S.abort_flag, S.timeout_ns, S.prof);
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<false>(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
+  solve_fp64<false>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
@@ -1008,15 +899,12 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
   Smem<float>& sm = solve_smem<float>();
   const int b0 = share(S.prob.M.nb, blockIdx.x, gridDim.x), b1 = share(S.prob.M.nb, blockIdx.x + 1, gridDim.x);
   const int r0 = share(S.prob.M.R, blockIdx.x, gridDim.x), r1 = share(S.prob.M.R, blockIdx.x + 1, gridDim.x);
-  GridBarrier B{S.bar, S.abort_flag, gridDim.x, globaltimer_ns() + S.timeout_ns, 0u, S.prof, globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = blockIdx.x;
-    sm.team_size = gridDim.x;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0) B.init(blockIdx.x, gridDim.x, S.bar, S.red, S.abort_flag, S.timeout_ns, S.prof);
   SineSolve<float> pin;
   pin.init();
   __syncthreads();
-  solve_mixed(sm, B, pin, S.prob, S.sp, S.red, b0, b1, r0, r1);
+  solve_mixed(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
 }
 
 // ========================================================= batches ========
@@ -1034,19 +922,16 @@ __device__ __forceinline__ void batch_body(const BatchArgs& A) {
   Smem<KT>& sm = solve_smem<KT>();
   const int team = A.team;
   const int g = blockIdx.x / team, rank = blockIdx.x % team;
-  GridBarrier B{A.bars + g, A.abort_flag, (unsigned)team, globaltimer_ns() + A.timeout_ns, 0u, A.prof,
-                globaltimer_ns()};
-  if (threadIdx.x == 0) {
-    sm.team_rank = rank;
-    sm.team_size = team;
-  }
+  Team& B = sm.team;
+  if (threadIdx.x == 0)
+    B.init((unsigned)rank, (unsigned)team, A.bars + g, A.red + (size_t)g * kRedWords * team, A.abort_flag, A.timeout_ns,
+           A.prof);
   SineSolve<KT> pin;
   pin.init();
   __syncthreads();
-  double* red = A.red + (size_t)g * kRedQ * team;
   while (true) {
     if (rank == 0 && threadIdx.x == 0) A.slots[g] = atomicAdd(A.queue, 1);
-    if (!B.sync(&sm.flag, 9)) return;
+    if (!B.sync(9)) return;
     unsigned long long t_begin = 0;
     if (threadIdx.x == 0) {
       t_begin = globaltimer_ns();
@@ -1061,12 +946,12 @@ __device__ __forceinline__ void batch_body(const BatchArgs& A) {
       const ProblemMixed& pr = A.pmx[p];
       const int b0 = share(pr.M.nb, rank, team), b1 = share(pr.M.nb, rank + 1, team);
       const int r0 = share(pr.M.R, rank, team), r1 = share(pr.M.R, rank + 1, team);
-      ok = solve_mixed(sm, B, pin, pr, A.sp, red, b0, b1, r0, r1);
+      ok = solve_mixed(sm, B, pin, pr, A.sp, b0, b1, r0, r1);
     } else {
       const Problem64& pr = A.p64[p];
       const int b0 = share(pr.M.nb, rank, team), b1 = share(pr.M.nb, rank + 1, team);
       const int r0 = share(pr.M.R, rank, team), r1 = share(pr.M.R, rank + 1, team);
-      ok = solve_fp64<false>(sm, B, pin, pr, A.sp, red, b0, b1, r0, r1);
+      ok = solve_fp64<false>(sm, B, pin, pr, A.sp, b0, b1, r0, r1);
     }
     if (!ok) return;
     if (rank == 0 && threadIdx.x == 0) {

@@ -319,7 +319,7 @@ int ensure_events(cup2d_poisson* h) {
 int ensure_scratch(cup2d_poisson* h) {
   int st;
   const int g = std::max(h->grid64, h->gridmx);
-  if ((st = h->red.ensure((int64_t)kRedQMean * std::max(g, 1))) || (st = h->bar.ensure(1)) ||
+  if ((st = h->red.ensure((int64_t)kRedWords * std::max(g, 1))) || (st = h->bar.ensure(1)) ||
       (st = h->abort_flag.ensure(1)) || (st = h->dstats.ensure(1)))
     return st;
   return CUP2D_OK;
@@ -1118,7 +1118,7 @@ int cup2d_batch_create(int32_t n, const cup2d_forest* forests, const cup2d_solve
                    [&](int32_t a, int32_t b) { return B->probs[a]->nb > B->probs[b]->nb; });
   const int gmax = std::max(B->grid64, B->gridmx);
   if ((st = B->d_p64.ensure(n)) || (st = B->d_pmx.ensure(n)) || (st = B->d_order.ensure(n)) ||
-      (st = B->red.ensure((int64_t)kRedQ * gmax)) || (st = B->bars.ensure(gmax)) || (st = B->slots.ensure(gmax)) ||
+      (st = B->red.ensure((int64_t)kRedWords * gmax)) || (st = B->bars.ensure(gmax)) || (st = B->slots.ensure(gmax)) ||
       (st = B->queue.ensure(1)) || (st = B->abort_flag.ensure(1)) || (st = B->dstats.ensure(n))) {
     cup2d_batch_destroy(B);
     return st;

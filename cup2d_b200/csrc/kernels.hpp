@@ -88,8 +88,6 @@ struct DevStats {
   unsigned long long t_begin, t_end;  // batch: globaltimer ns when the team took / finished the problem
 };
 
-constexpr int kRedQ = 20;      // reduction quantities per CTA
-constexpr int kRedQMean = 31;  // ... of the FP64 single solve with the mean constraint
 
 // One problem of a solve: its operator, right-hand side, FP64 solution and
 // best iterate, and the Krylov vectors (type T: FP64, or FP32 for the mixed
@@ -125,7 +123,7 @@ struct SolveParams {
 // and refer to the problem and parameters in place (no per-thread copies).
 struct SolveArgs64 {
   Problem64 prob;       // operator, b, x (x0 in, solution out), Krylov vectors
-  double* red;          // [kRedQ][grid]
+  double* red;          // [kRedWords * grid]
   unsigned* bar;        // arrival counter, zeroed before launch
   int* abort_flag;      // zeroed before launch
   SolveParams sp;
@@ -152,7 +150,7 @@ struct BatchArgs {
   const int32_t* order;     // [nprob] queue order
   int nprob;
   int team;                 // CTAs per problem; the grid is a multiple of it
-  double* red;              // [groups][kRedQ][team]
+  double* red;              // [groups][kRedWords * team]
   unsigned* bars;           // [groups] barrier counters, zeroed
   int* slots;               // [groups]
   int* queue;               // queue head, zeroed
@@ -162,7 +160,6 @@ struct BatchArgs {
   unsigned long long* prof;  // per-CTA phase timers, or null
 };
 
-constexpr int kSolveThreads = 256;
 // CTAs per SM of the persistent kernels (launch bounds and shared-memory
 // carve-out).  Single solves run 2 (128 registers): against 3 (80 registers,
 // spilling), on one box, time stepping 16.3 -> 18.3 solves/s (mixed) and
@@ -194,8 +191,8 @@ constexpr int kBatch64CtasPerSm = CUP2D_BATCH64_CTAS_PER_SM;
 // `served`: the server's instances (kServedCtasPerSm).
 int max_coop_grid_fp64(int device, bool served = false);
 int max_coop_grid_mixed(int device, bool served = false);
-// With a.sp.mean_row >= 0 the FP64 launch runs the mean-constraint variant
-// (its red holds kRedQMean quantities per CTA); the mixed form has none.
+// With a.sp.mean_row >= 0 the FP64 launch runs the mean-constraint variant;
+// the mixed form has none.
 cudaError_t launch_bicgstab64(const SolveArgs64& a, int grid, cudaStream_t s, bool served = false);
 cudaError_t launch_bicgstab_mixed(const SolveArgsMixed& a, int grid, cudaStream_t s, bool served = false);
 int max_coop_grid_mean(int device);

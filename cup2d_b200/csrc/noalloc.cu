@@ -54,7 +54,7 @@ constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 constexpr size_t kVecBytes = align256(sizeof(double) * kNoAllocMaxCells);
 constexpr size_t kOffVec = 0;  // xo, r, rh, p, nu, t, z, z2
 constexpr size_t kOffRed = kOffVec + 8 * kVecBytes;
-constexpr size_t kOffBar = kOffRed + align256(sizeof(double) * kRedQ * kNoAllocMaxGrid);
+constexpr size_t kOffBar = kOffRed + align256(sizeof(double) * kRedWords * kNoAllocMaxGrid);
 constexpr size_t kOffAbort = kOffBar + 256;
 constexpr size_t kOffStats = kOffAbort + 256;
 constexpr size_t kScratchBytes = kOffStats + align256(sizeof(DevStats));
