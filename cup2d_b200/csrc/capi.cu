@@ -204,6 +204,14 @@ struct cup2d_poisson {
     const int64_t want = (nb + blocks_per_cta - 1) / blocks_per_cta;
     return (int)std::max<int64_t>(1, std::min<int64_t>(want, maxg));
   }
+  // CTAs of the cluster that solves this forest, 0: the grid solver.  A forest
+  // that fits one cluster's shared memory is solved there, unless the caller
+  // chose a grid, asked for the grid solver's phase timers, or wants what only
+  // the grid solver has (the mean constraint; a server's own teams).
+  int cluster_for(bool mixed) const {
+    if (grid_override > 0 || profiling || served || opts.mean_constraint) return 0;
+    return mixed ? cluster_size<float>(device, nb) : cluster_size<double>(device, nb);
+  }
 };
 
 namespace {
@@ -454,6 +462,9 @@ int handle_create(const cup2d_forest* forest, const cup2d_solve_opts* opts, cuda
     cup2d_poisson_destroy(h);
     return CUP2D_CUDA_ERROR;
   }
+  // asks for the cluster solver's limits, which loads its kernels here and
+  // not in a solve that must not allocate
+  (void)cluster_size<double>(h->device, 1);
   if (const char* e = std::getenv("CUP2D_GRID")) h->grid_override = std::atoi(e);
   // the no-allocation solve's static scratch is committed here, with the
   // rest of the handle's memory, so that those solves never load or allocate
@@ -641,7 +652,31 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
   if (stats && (st = ensure_events(h))) return st;
   if (stats) cudaEventRecord(h->ev0, s);
   cudaError_t e;
-  if (o.precision == CUP2D_PREC_MIXED) {
+  const int cluster = h->cluster_for(mixed);
+  if (cluster > 0 && mixed) {
+    ClusterArgs<float> a{};
+    a.prob.M = h->mesh.view();
+    a.prob.b = d_b;
+    a.prob.x = d_x;
+    a.prob.xo = h->xo.p;
+    a.prob.stats = h->dstats.p;
+    a.abort_flag = h->abort_flag.p;
+    a.sp = SolveParams{o.tol_abs, o.tol_rel, o.reliable_delta, o.max_restarts, o.max_iter, o.subtract_mean,
+                       o.reliable_restart};
+    a.timeout_ns = tns;
+    e = launch_bicgstab_cluster(a, cluster, s);
+  } else if (cluster > 0) {
+    ClusterArgs<double> a{};
+    a.prob.M = h->mesh.view();
+    a.prob.b = d_b;
+    a.prob.x = d_x;
+    a.prob.xo = h->xo.p;
+    a.prob.stats = h->dstats.p;
+    a.abort_flag = h->abort_flag.p;
+    a.sp = SolveParams{o.tol_abs, o.tol_rel, 0.0, o.max_restarts, o.max_iter, o.subtract_mean, 0};
+    a.timeout_ns = tns;
+    e = launch_bicgstab_cluster(a, cluster, s);
+  } else if (mixed) {
     if ((st = ensure_mixed(h))) return st;
     SolveArgsMixed a{};
     a.prob = ProblemMixed{h->mesh.view(), d_b, d_x, h->xo.p, h->f_r.p, h->f_rh.p, h->f_p.p, h->f_nu.p,
@@ -1585,6 +1620,7 @@ int handle_view(const cup2d_poisson* h, HandleView* out) {
   out->M = h->mesh.view();
   out->nb = h->nb;
   out->grid = h->grid_for(h->grid64);
+  out->cluster = h->cluster_for(false);
   out->opts = h->opts;
   out->ev0 = h->ev0;
   out->ev1 = h->ev1;

@@ -62,6 +62,66 @@ __device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
 // residual read as converged)
 __device__ __forceinline__ double nanmax(double a, double b) { return (a > b || a != a) ? a : b; }
 
+// Maximum of non-negative (or NaN) values: their bits order like integers,
+// NaN above all.
+__device__ __forceinline__ double warp_max_nonneg(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(kFull, hi);
+  const unsigned ml = __reduce_max_sync(kFull, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+// The warp's partials of NV quantities into dst[0..NV): sums, and for bit q of
+// is_max set (a literal at every use) maxima of non-negative values.  Two sums
+// share their shuffles: a lane keeps one and hands the other over, so that
+// four sums take 6 exchanges, not 20 (a shuffle costs the SM a clock for every
+// warp: 40 a warp in the pass with four quantities).
+template <int NV>
+__device__ __forceinline__ void warp_partials(const double (&v)[NV], unsigned is_max, double* dst) {
+  const int lane = threadIdx.x & 31;
+  double s[NV + 3];
+  int at[NV + 3], n = 0;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    if ((is_max >> q) & 1u) {
+      const double m = warp_max_nonneg(v[q]);
+      if (lane == 0) dst[q] = m;
+    } else {
+      s[n] = v[q];
+      at[n++] = q;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; k += 4) {
+    if (k >= n) break;
+    const int m = n - k;  // sums left
+    double a, b = 0.0;
+    if (m == 1) {
+      a = s[k] + __shfl_xor_sync(kFull, s[k], 16);
+      a += __shfl_xor_sync(kFull, a, 8);
+    } else {
+      const bool up = (lane & 16) != 0;
+      a = (up ? s[k + 1] : s[k]) + __shfl_xor_sync(kFull, up ? s[k] : s[k + 1], 16);
+      if (m == 2) {
+        a += __shfl_xor_sync(kFull, a, 8);
+      } else {
+        const double c3 = m > 3 ? s[k + 3] : 0.0;
+        b = (up ? c3 : s[k + 2]) + __shfl_xor_sync(kFull, up ? s[k + 2] : c3, 16);
+        const bool up8 = (lane & 8) != 0;
+        a = (up8 ? b : a) + __shfl_xor_sync(kFull, up8 ? a : b, 8);
+      }
+    }
+    a += __shfl_xor_sync(kFull, a, 4);
+    a += __shfl_xor_sync(kFull, a, 2);
+    a += __shfl_xor_sync(kFull, a, 1);
+    // lanes 0, 16 hold sums k, k+1; lanes 8, 24 sums k+2, k+3
+    if (lane == 0) dst[at[k]] = a;
+    if (m > 1 && lane == 16) dst[at[k + 1]] = a;
+    if (m > 2 && lane == 8) dst[at[k + 2]] = a;
+    if (m > 3 && lane == 24) dst[at[k + 3]] = a;
+  }
+}
+
 constexpr int kSolveThreads = 256;
 constexpr int kWarps = kSolveThreads / 32;
 
@@ -229,17 +289,7 @@ struct Team {
   template <int NV>
   __device__ __forceinline__ bool reduce(const double (&v)[NV], unsigned is_max, int phase) {
     static_assert(NV <= kRedMax, "reduction slots");
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double r = v[q];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double b = __shfl_xor_sync(kFull, r, o);
-        r = ((is_max >> q) & 1u) ? nanmax(r, b) : r + b;
-      }
-      if (lane == 0) wred[w][q] = r;
-    }
+    warp_partials<NV>(v, is_max, wred[threadIdx.x >> 5]);
     return exchange(NV, is_max, phase);
   }
 };

@@ -14,7 +14,8 @@ struct HandleView {
   int device;                              // the handle's CUDA device
   MeshView M;                              // assembled operator (device)
   int64_t nb;                              // blocks
-  int grid;                                // CTAs the FP64 solve would use
+  int grid;                                // CTAs the FP64 solve would use,
+  int cluster;                             // or the CTAs of its cluster (0: a grid)
   cup2d_solve_opts opts;
   cudaEvent_t ev0, ev1;                    // the handle's timing events
 };

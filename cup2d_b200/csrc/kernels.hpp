@@ -187,6 +187,21 @@ constexpr int kBatchMixedCtasPerSm = CUP2D_BATCH_MIXED_CTAS_PER_SM;
 #endif
 constexpr int kBatch64CtasPerSm = CUP2D_BATCH64_CTAS_PER_SM;
 
+// A solve by one thread-block cluster (bicgstab_cluster.cu).
+template <class T>
+struct ClusterArgs {
+  Problem<T> prob;      // operator, b, x, xo and stats; the Krylov vectors live in shared memory
+  int* abort_flag;      // zeroed before launch
+  SolveParams sp;
+  unsigned long long timeout_ns;
+  int rows;             // explicit rows a CTA keeps in shared memory (set by the launch)
+};
+// CTAs of the cluster for a forest of nb blocks; 0: use the grid solver.
+template <class T>
+int cluster_size(int device, int64_t nb);
+template <class T>
+cudaError_t launch_bicgstab_cluster(ClusterArgs<T>& a, int size, cudaStream_t s);
+
 // Largest co-resident grid of the persistent kernels on this device.
 // `served`: the server's instances (kServedCtasPerSm).
 int max_coop_grid_fp64(int device, bool served = false);

@@ -6,7 +6,8 @@
 // memory is owned by its own pool allocator (the rest of the GPU is already
 // claimed), or a time-step loop that cannot afford the device-wide
 // synchronisation cudaMalloc/cudaFree can cause.  This entry point runs the
-// same FP64 persistent kernel (k_bicgstab64) with all of its scratch (eight
+// same FP64 persistent kernels (k_bicgstab64, or k_bicgstab64_cluster on a
+// forest that fits one cluster) with all of their scratch (eight
 // Krylov vectors, per-CTA reduction partials, the grid-barrier counter, the
 // abort flag and the statistics) in one file-scope
 // static device array, so the call itself allocates nothing: no cudaMalloc,
@@ -144,7 +145,17 @@ extern "C" int cup2d_poisson_solve_device_noalloc(cup2d_poisson* h, const double
   a.prof = nullptr;
 
   if (stats) cudaEventRecord(v.ev0, s);
-  const cudaError_t e = launch_bicgstab64(a, grid, s);
+  cudaError_t e;
+  if (v.cluster > 0) {  // small forests: one cluster, as the allocating solve
+    ClusterArgs<double> c{};
+    c.prob = a.prob;
+    c.abort_flag = a.abort_flag;
+    c.sp = a.sp;
+    c.timeout_ns = a.timeout_ns;
+    e = launch_bicgstab_cluster(c, v.cluster, s);
+  } else {
+    e = launch_bicgstab64(a, grid, s);
+  }
   if (e != cudaSuccess) return e == cudaErrorNoDevice ? CUP2D_NO_DEVICE : CUP2D_CUDA_ERROR;
   if (!stats) return CUP2D_OK;
   cudaEventRecord(v.ev1, s);

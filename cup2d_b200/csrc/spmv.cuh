@@ -133,6 +133,18 @@ __device__ __forceinline__ void lds16(const T* p, T (&v)[N]) {
   }
 }
 
+// Two consecutive values from shared memory (p aligned to the pair).
+template <class T>
+__device__ __forceinline__ void lds_pair(const T* p, T (&v)[2]) {
+  if constexpr (sizeof(T) == 4) {
+    const float2 a = *reinterpret_cast<const float2*>(p);
+    v[0] = a.x; v[1] = a.y;
+  } else {
+    const double2 a = *reinterpret_cast<const double2*>(p);
+    v[0] = a.x; v[1] = a.y;
+  }
+}
+
 template <int N, class T>
 __device__ __forceinline__ void stv(T* p, const T (&v)[N]) {
   static_assert(N * sizeof(T) % 8 == 0, "vector size");
