@@ -38,10 +38,12 @@ __device__ __forceinline__ unsigned long long explicit_mask(const MeshView& M, i
   return 0ull;
 }
 
-// Entries of an explicit row whose loads are issued as one batch: 8 in FP32,
-// 4 in FP64 (whose batch kernels run at 80 registers a thread).
+// Entries of an explicit row whose loads are issued as one batch.  Rows hold
+// 7, 8 or 9 entries (9: 16 % of them, so nearly every warp has one; 1 % hold
+// 13).  With 8 (FP32) and 4 (FP64) the rest took two more round trips: us in
+// pass B at 1,500 blocks FP64 2.9 -> 2.6, at 128 blocks 3.3 -> 2.7.
 template <class T>
-constexpr int kRowBatch = sizeof(T) == 4 ? 8 : 4;
+constexpr int kRowBatch = 9;
 
 // sum_k vals[k] z[xcol[k]] of an explicit row, k ascending over [k0, k1).
 // The columns and values of the first kRowBatch entries are requested
