@@ -46,7 +46,8 @@ namespace cup2d {
 
 namespace {
 
-constexpr int kProjThreads = 256;  // 4 blocks of 64 cells per CTA
+constexpr int kProjThreads = 256;  // 8 warps, a block of 64 cells each at a time
+constexpr int kProjWarps = kProjThreads / 32;
 constexpr double kI23 = 2. / 3., kI15 = 1. / 5., kI815 = 8. / 15.;
 
 enum : int { kSame = 0, kEdge = 1, kCoarser = 2, kFiner = 3 };
@@ -233,235 +234,258 @@ __device__ __forceinline__ double grad_face(int f, double pFac, double g, double
   return ((f & 1) == 0 ? pFac : -pFac) * (g + w);
 }
 
-// Labs in shared memory: kLabBlocks blocks per CTA, 64 threads each.  Every
-// thread stages its cell; 32 threads of each block then fill the ghost
-// layer (the face neighbours, the edge rules, the coarse/fine rules) and, on
-// faces with finer neighbours, the flux-correction terms; then every thread
-// evaluates its cell from shared memory.  The stencil threads stay simple,
-// the irregular work is confined to the ghost threads.
-constexpr int kLabBlocks = kProjThreads / kBLEN;
-constexpr int kLab = kBS + 2;
-enum : int { kLabU = 0, kLabV = 1, kLabUd = 2, kLabVd = 3, kLabP = 4, kLabs = 5 };
+// One warp per block: lane l holds cells l and l + 32 (rows l / 8 and l / 8 + 4,
+// column l % 8), and the block's 32 ghosts are one a lane (face l / 8, position
+// l % 8 along it).  A warp's loads of a block, its own cells and its ghosts, go
+// out together (the faces' table entries are read one block ahead), and the
+// stencil's neighbours come by shuffles: no shared memory, no CTA barrier, so
+// an SM keeps all its warps' loads in flight.  Four blocks to a CTA with labs in
+// shared memory waited at a CTA barrier for the slowest ghost's dependent loads;
+// labs of one warp each were bound by the L1/shared-memory pipe (79-86 % busy,
+// lab rows and interleaved pairs conflicting).  us on 1.15 M blocks (73 M cells),
+// CTA labs -> warp labs -> shuffles: right-hand side and the reset of pres 1833
+// -> 1686 -> 1393 (3.4 TB/s), correction 1028 -> 724 -> 585 (5.0 TB/s); on 0.1 M blocks
+// 225 -> 206 -> 172 and 127 -> 89 -> 77.  Bound now by the ghosts' scattered sectors.
 
-struct ProjSmem {
-  double lab[kLabs][kLabBlocks][kLab][kLab];
-  double corr[2][kLabBlocks][4][kBS];  // finer faces: [0] divergence / gradient, [1] Laplacian
-  int kind[kLabBlocks][4];
+// The neighbours of a lane's two values a0 (cell l), a1 (cell l + 32): across
+// the block's faces the ghosts g of the other lanes.
+struct Around {
+  double w[2], e[2], s[2], n[2];
 };
+__device__ __forceinline__ double from_lane(double v, int src) { return __shfl_sync(kFull, v, src & 31); }
 
-__device__ __forceinline__ double& labv(ProjSmem& S, int q, int lb, int ix, int iy) {
-  return S.lab[q][lb][iy + 1][ix + 1];
+__device__ __forceinline__ void around_x(int lane, double a0, double a1, double g, Around& o) {
+  const int r = lane >> 3, c = lane & 7;
+  const int src = c == 7 ? 8 + r : r;  // column 0 takes the W ghosts of its rows, column 7 the E ghosts
+  const double g0 = from_lane(g, src), g1 = from_lane(g, src + 4);
+  const double w0 = from_lane(a0, lane - 1), w1 = from_lane(a1, lane - 1);
+  const double e0 = from_lane(a0, lane + 1), e1 = from_lane(a1, lane + 1);
+  o.w[0] = c > 0 ? w0 : g0;
+  o.w[1] = c > 0 ? w1 : g1;
+  o.e[0] = c < 7 ? e0 : g0;
+  o.e[1] = c < 7 ? e1 : g1;
+}
+__device__ __forceinline__ void around_y(int lane, double a0, double a1, double g, Around& o) {
+  const int r = lane >> 3, c = lane & 7;
+  const double gg = from_lane(g, (r == 3 ? 24 : 16) + c);  // row 0 takes the S ghosts, row 7 the N ghosts
+  const double n0 = from_lane(a0, lane + 8), n1 = from_lane(a1, lane + 8);
+  const double s0 = from_lane(a0, lane - 8), s1 = from_lane(a1, lane - 8);
+  o.s[0] = r > 0 ? s0 : gg;
+  o.n[0] = r < 3 ? n0 : n1;  // row 3 -> row 4
+  o.s[1] = r > 0 ? s1 : s0;  // row 4 -> row 3
+  o.n[1] = r < 3 ? n1 : gg;
 }
 
-// What one thread loads for its cell of a group of kLabBlocks blocks, one
-// group ahead of the group it computes: the staged values and, for ghost
-// threads, the face's neighbour table entry.  CTAs are persistent: each
-// walks groups blockIdx.x, + gridDim.x, ..., so the loads of the next group
-// are in flight while the ghost work and the stencil of the current one run.
-struct Prefetch {
-  double2 u, ud;
-  double chi, p;
-  int32_t code;
+// Whether each of a block's faces has finer neighbours (bit f), from its
+// lanes' sides.
+__device__ __forceinline__ unsigned finer_faces(int kind) {
+  const unsigned m = __ballot_sync(kFull, kind == kFiner);
+  return (m & 1u) | ((m >> 7) & 2u) | ((m >> 14) & 4u) | ((m >> 21) & 8u);
+}
+
+// The flux corrections (one a ghost lane, on finer faces) at a lane's two
+// cells: across x (faces W, E) and across y (face S of cell l, N of cell l + 32).
+struct FluxAt {
+  double x[2], y;
+  bool w, e, s, n;
+  __device__ __forceinline__ FluxAt(int lane, unsigned finer, double corr) {
+    const int r = lane >> 3, c = lane & 7;
+    const int src = c == 7 ? 8 + r : r;
+    x[0] = from_lane(corr, src);
+    x[1] = from_lane(corr, src + 4);
+    y = from_lane(corr, (r == 3 ? 24 : 16) + c);
+    w = c == 0 && (finer & 1u);
+    e = c == 7 && (finer & 2u);
+    s = r == 0 && (finer & 4u);
+    n = r == 3 && (finer & 8u);
+  }
 };
 
-// The RHS kernel's labs, double-buffered: the next group's cells are copied
-// in with cp.async (16-byte (u, v) pairs straight into shared memory, no
-// registers held) while the current group is computed.
-struct RhsSmem {
-  double2 uv[2][kLabBlocks][kLab][kLab];  // (u, v); a face's ghost fills the normal component only
-  double2 ud[2][kLabBlocks][kLab][kLab];  // (ud, vd)
-  double p[2][kLabBlocks][kLab][kLab];
-  double chi[2][kLabBlocks][kBLEN];
-  double corr[2][kLabBlocks][4][kBS];     // finer faces: [0] divergence, [1] Laplacian
-  int kind[kLabBlocks][4];
-};
-
-__global__ void __launch_bounds__(kProjThreads, 4) k_pressure_rhs(const __grid_constant__ Geo G, double dt,
+__global__ void __launch_bounds__(kProjThreads, 3) k_pressure_rhs(const __grid_constant__ Geo G, double dt,
                                                                     const __grid_constant__ ProjFields P) {
-  __shared__ __align__(16) RhsSmem S;
-  const int lb = threadIdx.x >> 6, c = threadIdx.x & 63, ix = c & 7, iy = c >> 3;
+  const int lane = threadIdx.x & 31;
   const bool vel = P.vel != nullptr, pres = P.pres != nullptr;
-  // ghost work: threads 0-31 of a block the velocity ghosts, 32-63 the
-  // pressure ghosts (ghost index c % 32)
-  const int gi = c & 31;
-  const bool gvel = c < 32 && vel, gpres = c >= 32 && pres, gthr = gvel || gpres;
-  const int64_t ngroups = (G.F.nb + kLabBlocks - 1) / kLabBlocks;
-  // copies of group grp's cells into buffer q, and the face's table entry
-  auto issue = [&](int64_t grp, int q, int32_t& code) {
-    const int64_t b = grp * kLabBlocks + lb;
-    if (b >= G.F.nb) return;
-    const int64_t cell = b * kBLEN + c;
-    if (vel) {
-      cp_async_n<16>(&S.uv[q][lb][iy + 1][ix + 1], P.vel + 2 * cell, 16);
-      cp_async_n<16>(&S.ud[q][lb][iy + 1][ix + 1], P.udef + 2 * cell, 16);
-      cp_async_n<8>(&S.chi[q][lb][c], P.chi + cell, 8);
-    }
-    if (pres) cp_async_n<8>(&S.p[q][lb][iy + 1][ix + 1], P.pres + cell, 8);
-    if (gthr) code = __ldg(G.nbr + 4 * b + (gi >> 3));
-  };
-  int32_t code = 0, code_next = 0;
-  int64_t grp = blockIdx.x;
-  if (grp < ngroups) issue(grp, 0, code);
-  cp_async_commit_group();
-  for (int it = 0; grp < ngroups; grp += gridDim.x, ++it) {
-    const int q = it & 1;
-    cp_async_wait_n<0>();  // this group's cells have landed (every thread's, after the barrier)
-    __syncthreads();
-    if (grp + gridDim.x < ngroups) issue(grp + gridDim.x, q ^ 1, code_next);
-    cp_async_commit_group();
-    const int64_t b = grp * kLabBlocks + lb;
-    const bool valid = b < G.F.nb;
-    const int64_t cell = b * kBLEN + c;
-    // ghost layer and flux-correction terms
-    if (valid && gthr) {
-      const Ghost gh(G, b, gi, G.side_from_code(b, gi >> 3, code));
-      const int k = gi & 7, f = gh.f;
-      if (k == 0 && (c < 32 || !vel)) S.kind[lb][f] = gh.s.kind;
-      const int gx = gh.ix + (f == 0 ? -1 : f == 1 ? 1 : 0), gy = gh.iy + (f == 2 ? -1 : f == 3 ? 1 : 0);
-      const double h = cell_h(G.F, G.F.level[b]);
-      if (gvel) {
-        const Fld V{P.vel, 2}, U{P.udef, 2};
-        const int cmp = gh.xface() ? 0 : 1;  // the normal component: the only one the divergence reads
-        const double g = gh.value(V, cmp, true), gd = gh.value(U, cmp, true);
-        if (cmp == 0) {
-          S.uv[q][lb][gy + 1][gx + 1].x = g;
-          S.ud[q][lb][gy + 1][gx + 1].x = gd;
-        } else {
-          S.uv[q][lb][gy + 1][gx + 1].y = g;
-          S.ud[q][lb][gy + 1][gx + 1].y = gd;
-        }
-        if (gh.s.kind == kFiner) {
-          const double facDiv = 0.5 * h / dt;
-          const double own =
-              div_face(f, facDiv, __ldg(P.chi + gh.cell), g, V.v(gh.cell, cmp), gd, U.v(gh.cell, cmp));
-          int64_t fb;
-          int k0;
-          gh.fine_cells(fb, k0);
-          const double facDivF = 0.5 * cell_h(G.F, G.F.level[fb]) / dt;
-          double fs[2];
-          for (int r = 0; r < 2; ++r) {
-            const int64_t fc = gh.fine_cell(fb, k0, r, 0);
-            fs[r] = div_face(f ^ 1, facDivF, __ldg(P.chi + fc), gh.fine_ghost(V, cmp, fb, k0, r), V.v(fc, cmp),
-                             gh.fine_ghost(U, cmp, fb, k0, r), U.v(fc, cmp));
-          }
-          S.corr[0][lb][f][k] = own + (fs[0] + fs[1]);
-        }
-      }
-      if (gpres) {
-        const Fld Q{P.pres, 1};
-        const double g = gh.value(Q, 0, false);
-        S.p[q][lb][gy + 1][gx + 1] = g;
-        if (gh.s.kind == kFiner) {
-          const double own = g - Q.v(gh.cell, 0);
-          int64_t fb;
-          int k0;
-          gh.fine_cells(fb, k0);
-          double fs[2];
-          for (int r = 0; r < 2; ++r) fs[r] = gh.fine_ghost(Q, 0, fb, k0, r) - Q.v(gh.fine_cell(fb, k0, r, 0), 0);
-          S.corr[1][lb][f][k] = own + (fs[0] + fs[1]);
-        }
-      }
-    }
-    __syncthreads();
-    if (valid) {
-      const bool edge[4] = {ix == 0, ix == kBS - 1, iy == 0, iy == kBS - 1};
-      const int along[4] = {iy, iy, ix, ix};
-      const int X = ix + 1, Y = iy + 1;
-      double t;
+  const int f = lane >> 3;
+  const int64_t step = (int64_t)gridDim.x * kProjWarps;
+  int64_t b = (int64_t)blockIdx.x * kProjWarps + (threadIdx.x >> 5);
+  int32_t code = 0, level = 0;
+  if (b < G.F.nb) {
+    code = __ldg(G.nbr + 4 * b + f);
+    level = __ldg(G.F.level + b);
+  }
+  for (; b < G.F.nb; b += step) {
+    const int64_t cell = b * kBLEN + lane;
+    const Fld V{P.vel, 2}, U{P.udef, 2}, Q{P.pres, 1};
+    double2 u[2], ud[2];
+    double chi[2], p[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
       if (vel) {
-        const double h = cell_h(G.F, G.F.level[b]);
-        const double facDiv = 0.5 * h / dt;
-        const double chi = S.chi[q][lb][c];
-        t = facDiv * ((S.uv[q][lb][Y][X + 1].x - S.uv[q][lb][Y][X - 1].x) +
-                      (S.uv[q][lb][Y + 1][X].y - S.uv[q][lb][Y - 1][X].y));
-        t += -facDiv * chi * ((S.ud[q][lb][Y][X + 1].x - S.ud[q][lb][Y][X - 1].x) +
-                              (S.ud[q][lb][Y + 1][X].y - S.ud[q][lb][Y - 1][X].y));
-        for (int f = 0; f < 4; ++f)
-          if (edge[f] && S.kind[lb][f] == kFiner) t = t + S.corr[0][lb][f][along[f]];
-      } else {
-        t = P.tmp[cell];
+        u[j] = __ldg(reinterpret_cast<const double2*>(P.vel) + cell + 32 * j);
+        ud[j] = __ldg(reinterpret_cast<const double2*>(P.udef) + cell + 32 * j);
+        chi[j] = __ldg(P.chi + cell + 32 * j);
+      }
+      if (pres) p[j] = P.pres[cell + 32 * j];
+    }
+    const Ghost gh(G, b, lane, G.side_from_code(b, f, code));
+    const unsigned finer = finer_faces(gh.s.kind);
+    const double h = cell_h(G.F, level);
+    const double facDiv = 0.5 * h / dt;
+    const int cmp = gh.xface() ? 0 : 1;  // the normal component: the only one the divergence reads
+    double g = 0.0, gd = 0.0, gp = 0.0;
+    if (vel) {
+      g = gh.value(V, cmp, true);
+      gd = gh.value(U, cmp, true);
+    }
+    if (pres) gp = gh.value(Q, 0, false);
+    // the next block's faces
+    const int64_t bn = b + step;
+    if (bn < G.F.nb) {
+      code = __ldg(G.nbr + 4 * bn + f);
+      level = __ldg(G.F.level + bn);
+    }
+    double corr[2] = {0.0, 0.0};  // flux corrections: divergence, Laplacian
+    if (gh.s.kind == kFiner) {
+      int64_t fb;
+      int k0;
+      gh.fine_cells(fb, k0);
+      if (vel) {
+        const double own = div_face(f, facDiv, __ldg(P.chi + gh.cell), g, V.v(gh.cell, cmp), gd, U.v(gh.cell, cmp));
+        const double facDivF = 0.5 * cell_h(G.F, G.F.level[fb]) / dt;
+        double fs[2];
+        for (int r = 0; r < 2; ++r) {
+          const int64_t fc = gh.fine_cell(fb, k0, r, 0);
+          fs[r] = div_face(f ^ 1, facDivF, __ldg(P.chi + fc), gh.fine_ghost(V, cmp, fb, k0, r), V.v(fc, cmp),
+                           gh.fine_ghost(U, cmp, fb, k0, r), U.v(fc, cmp));
+        }
+        corr[0] = own + (fs[0] + fs[1]);
       }
       if (pres) {
-        const double p0 = S.p[q][lb][Y][X];
-        t -= ((S.p[q][lb][Y][X - 1] + S.p[q][lb][Y][X + 1]) + (S.p[q][lb][Y - 1][X] + S.p[q][lb][Y + 1][X])) -
-             4.0 * p0;
-        for (int f = 0; f < 4; ++f)
-          if (edge[f] && S.kind[lb][f] == kFiner) t = t + S.corr[1][lb][f][along[f]];
-        P.pold[cell] = p0;
+        const double own = gp - Q.v(gh.cell, 0);
+        double fs[2];
+        for (int r = 0; r < 2; ++r) fs[r] = gh.fine_ghost(Q, 0, fb, k0, r) - Q.v(gh.fine_cell(fb, k0, r, 0), 0);
+        corr[1] = own + (fs[0] + fs[1]);
       }
-      P.tmp[cell] = t;
     }
-    code = code_next;
-    // the next iteration's first barrier orders these reads of buffer q
-    // before that iteration's copies into it
+    __syncwarp();
+    double t[2];
+    if (vel) {
+      Around a, d;
+      around_x(lane, u[0].x, u[1].x, g, a);
+      around_y(lane, u[0].y, u[1].y, g, a);
+      around_x(lane, ud[0].x, ud[1].x, gd, d);
+      around_y(lane, ud[0].y, ud[1].y, gd, d);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        t[j] = facDiv * ((a.e[j] - a.w[j]) + (a.n[j] - a.s[j]));
+        t[j] += -facDiv * chi[j] * ((d.e[j] - d.w[j]) + (d.n[j] - d.s[j]));
+      }
+      if (finer) {  // in face order
+        const FluxAt q(lane, finer, corr[0]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (q.w) t[j] = t[j] + q.x[j];
+          if (q.e) t[j] = t[j] + q.x[j];
+        }
+        if (q.s) t[0] = t[0] + q.y;
+        if (q.n) t[1] = t[1] + q.y;
+      }
+    } else {
+      t[0] = P.tmp[cell];
+      t[1] = P.tmp[cell + 32];
+    }
+    if (pres) {
+      Around a;
+      around_x(lane, p[0], p[1], gp, a);
+      around_y(lane, p[0], p[1], gp, a);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) t[j] -= ((a.w[j] + a.e[j]) + (a.s[j] + a.n[j])) - 4.0 * p[j];
+      if (finer) {
+        const FluxAt q(lane, finer, corr[1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (q.w) t[j] = t[j] + q.x[j];
+          if (q.e) t[j] = t[j] + q.x[j];
+        }
+        if (q.s) t[0] = t[0] + q.y;
+        if (q.n) t[1] = t[1] + q.y;
+      }
+      P.pold[cell] = p[0];
+      P.pold[cell + 32] = p[1];
+    }
+    P.tmp[cell] = t[0];
+    P.tmp[cell + 32] = t[1];
   }
-  cp_async_wait_n<0>();  // nothing may land after return
 }
 
 __global__ void __launch_bounds__(kProjThreads, 4) k_pressure_correction(const __grid_constant__ Geo G, double dt,
                                                                            const double* __restrict__ pres,
                                                                            double* __restrict__ vel) {
-  __shared__ ProjSmem S;
-  const int lb = threadIdx.x >> 6, c = threadIdx.x & 63, ix = c & 7, iy = c >> 3;
-  const bool gthr = c < 4 * kBS;
+  const int lane = threadIdx.x & 31;
   const Fld Q{pres, 1};
-  const int64_t ngroups = (G.F.nb + kLabBlocks - 1) / kLabBlocks;
-  auto fetch = [&](int64_t grp, Prefetch& q) {
-    const int64_t b = grp * kLabBlocks + lb;
-    if (b >= G.F.nb) return;
-    const int64_t cell = b * kBLEN + c;
-    q.p = __ldg(pres + cell);
-    q.u = reinterpret_cast<const double2*>(vel)[cell];  // updated in place: no read-only path
-    if (gthr) q.code = __ldg(G.nbr + 4 * b + (c >> 3));
-  };
-  Prefetch cur{}, nxt{};
-  int64_t grp = blockIdx.x;
-  if (grp < ngroups) fetch(grp, cur);
-  for (; grp < ngroups; grp += gridDim.x) {
-    const int64_t b = grp * kLabBlocks + lb;
-    const bool valid = b < G.F.nb;
-    const int64_t cell = b * kBLEN + c;
-    if (valid) labv(S, kLabP, lb, ix, iy) = cur.p;
-    if (grp + gridDim.x < ngroups) fetch(grp + gridDim.x, nxt);
-    if (valid && gthr) {
-      const Ghost gh(G, b, c, G.side_from_code(b, c >> 3, cur.code));
-      const int k = c & 7, f = gh.f;
-      if (k == 0) S.kind[lb][f] = gh.s.kind;
-      const int gx = gh.ix + (f == 0 ? -1 : f == 1 ? 1 : 0), gy = gh.iy + (f == 2 ? -1 : f == 3 ? 1 : 0);
-      const double g = gh.value(Q, 0, false);
-      labv(S, kLabP, lb, gx, gy) = g;
-      if (gh.s.kind == kFiner) {
-        const double pFac = -0.5 * dt * cell_h(G.F, G.F.level[b]);
-        const double own = grad_face(f, pFac, g, Q.v(gh.cell, 0));
-        int64_t fb;
-        int k0;
-        gh.fine_cells(fb, k0);
-        const double pFacF = -0.5 * dt * cell_h(G.F, G.F.level[fb]);
-        double fs[2];
-        for (int q = 0; q < 2; ++q)
-          fs[q] = grad_face(f ^ 1, pFacF, gh.fine_ghost(Q, 0, fb, k0, q), Q.v(gh.fine_cell(fb, k0, q, 0), 0));
-        S.corr[0][lb][f][k] = own + (fs[0] + fs[1]);
+  const int f = lane >> 3;
+  const int64_t step = (int64_t)gridDim.x * kProjWarps;
+  int64_t b = (int64_t)blockIdx.x * kProjWarps + (threadIdx.x >> 5);
+  int32_t code = 0, level = 0;
+  if (b < G.F.nb) {
+    code = __ldg(G.nbr + 4 * b + f);
+    level = __ldg(G.F.level + b);
+  }
+  for (; b < G.F.nb; b += step) {
+    const int64_t cell = b * kBLEN + lane;
+    const double p[2] = {__ldg(pres + cell), __ldg(pres + cell + 32)};
+    double2 v[2];  // updated in place: no read-only path
+#pragma unroll
+    for (int j = 0; j < 2; ++j) v[j] = reinterpret_cast<const double2*>(vel)[cell + 32 * j];
+    const Ghost gh(G, b, lane, G.side_from_code(b, f, code));
+    const unsigned finer = finer_faces(gh.s.kind);
+    const double h = cell_h(G.F, level);
+    const double pFac = -0.5 * dt * h;
+    const double g = gh.value(Q, 0, false);
+    const int64_t bn = b + step;
+    if (bn < G.F.nb) {
+      code = __ldg(G.nbr + 4 * bn + f);
+      level = __ldg(G.F.level + bn);
+    }
+    double corr = 0.0;
+    if (gh.s.kind == kFiner) {
+      const double own = grad_face(f, pFac, g, Q.v(gh.cell, 0));
+      int64_t fb;
+      int k0;
+      gh.fine_cells(fb, k0);
+      const double pFacF = -0.5 * dt * cell_h(G.F, G.F.level[fb]);
+      double fs[2];
+      for (int q = 0; q < 2; ++q)
+        fs[q] = grad_face(f ^ 1, pFacF, gh.fine_ghost(Q, 0, fb, k0, q), Q.v(gh.fine_cell(fb, k0, q, 0), 0));
+      corr = own + (fs[0] + fs[1]);
+    }
+    __syncwarp();
+    Around a;
+    around_x(lane, p[0], p[1], g, a);
+    around_y(lane, p[0], p[1], g, a);
+    double tx[2], ty[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      tx[j] = pFac * (a.e[j] - a.w[j]);
+      ty[j] = pFac * (a.n[j] - a.s[j]);
+    }
+    if (finer) {
+      const FluxAt q(lane, finer, corr);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (q.w) tx[j] = tx[j] + q.x[j];
+        if (q.e) tx[j] = tx[j] + q.x[j];
       }
+      if (q.s) ty[0] = ty[0] + q.y;
+      if (q.n) ty[1] = ty[1] + q.y;
     }
-    __syncthreads();
-    if (valid) {
-      const double h = cell_h(G.F, G.F.level[b]);
-      const double pFac = -0.5 * dt * h;
-      double tv[2];
-      tv[0] = pFac * (labv(S, kLabP, lb, ix + 1, iy) - labv(S, kLabP, lb, ix - 1, iy));
-      tv[1] = pFac * (labv(S, kLabP, lb, ix, iy + 1) - labv(S, kLabP, lb, ix, iy - 1));
-      const bool edge[4] = {ix == 0, ix == kBS - 1, iy == 0, iy == kBS - 1};
-      const int along[4] = {iy, iy, ix, ix};
-      for (int f = 0; f < 4; ++f)
-        if (edge[f] && S.kind[lb][f] == kFiner) tv[f < 2 ? 0 : 1] = tv[f < 2 ? 0 : 1] + S.corr[0][lb][f][along[f]];
-      const double ih2 = 1.0 / h / h;
-      double2 v = cur.u;
-      v.x += tv[0] * ih2;
-      v.y += tv[1] * ih2;
-      reinterpret_cast<double2*>(vel)[cell] = v;
+    const double ih2 = 1.0 / h / h;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      v[j].x += tx[j] * ih2;
+      v[j].y += ty[j] * ih2;
+      reinterpret_cast<double2*>(vel)[cell + 32 * j] = v[j];
     }
-    __syncthreads();
-    cur = nxt;
   }
 }
 
@@ -487,7 +511,7 @@ int persistent_grid(const void* fn, int which, int64_t ngroups) {
 cudaError_t launch_pressure_rhs(const ForestView& F, const int32_t* nbr, double dt, const ProjFields& f,
                                 cudaStream_t s) {
   if (F.nb <= 0) return cudaSuccess;
-  const int grid = persistent_grid((const void*)k_pressure_rhs, 0, (F.nb + kLabBlocks - 1) / kLabBlocks);
+  const int grid = persistent_grid((const void*)k_pressure_rhs, 0, (F.nb + kProjWarps - 1) / kProjWarps);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   k_pressure_rhs<<<grid, kProjThreads, 0, s>>>(Geo{F, nbr}, dt, f);
   return cudaGetLastError();
@@ -496,7 +520,7 @@ cudaError_t launch_pressure_rhs(const ForestView& F, const int32_t* nbr, double 
 cudaError_t launch_pressure_correction(const ForestView& F, const int32_t* nbr, double dt, const double* pres,
                                        double* vel, cudaStream_t s) {
   if (F.nb <= 0) return cudaSuccess;
-  const int grid = persistent_grid((const void*)k_pressure_correction, 1, (F.nb + kLabBlocks - 1) / kLabBlocks);
+  const int grid = persistent_grid((const void*)k_pressure_correction, 1, (F.nb + kProjWarps - 1) / kProjWarps);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   k_pressure_correction<<<grid, kProjThreads, 0, s>>>(Geo{F, nbr}, dt, pres, vel);
   return cudaGetLastError();
