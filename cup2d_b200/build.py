@@ -18,7 +18,7 @@ BUILD = PKG / "_build"
 LIB = PKG / "libcup2d_poisson.so"
 
 SOURCES = ["assemble.cu", "adapt.cu", "bicgstab.cu", "bicgstab_cluster.cu", "capi.cu", "noalloc.cu", "precond_tc.cu", "projection.cu",
-           "server.cu", "timestep.cu", "spmv_staged.cu", "problems.cpp", "forest.cpp"]
+           "server.cu", "timestep.cu", "spmv_apply.cu", "problems.cpp", "forest.cpp"]
 # files whose arithmetic must round like a plain IEEE evaluation (no FMA)
 FILE_FLAGS = {"projection.cu": ["--fmad=false"]}
 HEADERS = ["common.cuh", "kernels.hpp", "spmv.cuh", "sine_solve.cuh", "handle_view.hpp", "forest.hpp"]

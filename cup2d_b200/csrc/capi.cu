@@ -737,13 +737,13 @@ int cup2d_poisson_solve(cup2d_poisson* h, const double* b, double* x, cup2d_solv
 int cup2d_poisson_apply(cup2d_poisson* h, const double* d_x, double* d_y, void* stream) {
   if (!h || !d_x || !d_y || !aligned16(d_x) || !aligned16(d_y)) return CUP2D_INVALID_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the legacy default stream
-  return from_cuda(launch_spmv64(h->mesh.view(), d_x, d_y, h->err.p, s));
+  return from_cuda(launch_spmv64(h->mesh.view(), d_x, d_y, s));
 }
 
 int cup2d_poisson_apply32(cup2d_poisson* h, const float* d_x, float* d_y, void* stream) {
   if (!h || !d_x || !d_y || !aligned16(d_x) || !aligned16(d_y)) return CUP2D_INVALID_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the legacy default stream
-  return from_cuda(launch_spmv32(h->mesh.view(), d_x, d_y, h->err.p, s));
+  return from_cuda(launch_spmv32(h->mesh.view(), d_x, d_y, s));
 }
 
 }  // extern "C"

@@ -215,9 +215,9 @@ int max_coop_grid_batch(int device, bool mixed);
 cudaError_t launch_bicgstab_batch(const BatchArgs& a, int grid, bool mixed, cudaStream_t s);
 
 // Single operations (tests, residual checks).
-// y = A x (spmv_staged.cu); *err raised if a staged copy did not complete.
-cudaError_t launch_spmv64(const MeshView& M, const double* x, double* y, int* err, cudaStream_t s);
-cudaError_t launch_spmv32(const MeshView& M, const float* x, float* y, int* err, cudaStream_t s);
+// y = A x (spmv_apply.cu).
+cudaError_t launch_spmv64(const MeshView& M, const double* x, double* y, cudaStream_t s);
+cudaError_t launch_spmv32(const MeshView& M, const float* x, float* y, cudaStream_t s);
 cudaError_t launch_precond64(const double* P, int64_t nb, const double* p, double* z, cudaStream_t s);
 cudaError_t launch_precond32(const float* P32, int64_t nb, const float* p, float* z, cudaStream_t s);
 // The same apply on tcgen05 tensor cores with TMEM accumulators (precond_tc.cu).
