@@ -21,6 +21,12 @@
 //            interleaved) marks a dense key array, an exclusive scan of which
 //            gives each leaf its position: the leaves in Morton order.
 //
+// One cooperative launch does all of it up to the ranks, with a grid barrier
+// between the steps (about 1 us; some forty of them), a second writes the leaves
+// once the host has sized their arrays.  As a launch per level and step it was
+// some ninety launches and a host round trip per balance round.  Remesh of the
+// 20,834-block forest (adaptation, assembly, read-back, transfer): 877 -> 560 us.
+//
 // The result is the forest the host generator builds for the same geometry
 // (forest.cpp build_disk_forest: same geometric test with the same rounded
 // operations, same balance rule, same order); the device assembly and the
@@ -35,6 +41,8 @@
 namespace cup2d {
 
 namespace {
+
+constexpr int kAdaptThreads = 1024;  // one CTA an SM
 
 constexpr uint8_t kAbsent = 0, kLeaf = 1, kRefined = 2, kSplit = 3;  // kSplit: a leaf marked for splitting
 
@@ -54,16 +62,20 @@ __device__ __forceinline__ bool meets_band(double x0, double y0, double x1, doub
   return dmin <= __dadd_rn(r, band) && dmax >= __dadd_rn(r, -band);
 }
 
-__global__ void k_adapt_tag(const __grid_constant__ AdaptGeom g, const __grid_constant__ AdaptDisks D, int l,
-                            uint8_t* __restrict__ state) {
+// Positions of a level are shared out over the threads of the grid.  States
+// that other CTAs wrote before a grid barrier are read from L2.
+__device__ __forceinline__ int64_t grid_thread() { return blockIdx.x * (int64_t)blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int64_t grid_threads() { return (int64_t)gridDim.x * blockDim.x; }
+
+__device__ __forceinline__ void adapt_tag(const AdaptGeom& g, const AdaptDisks& D, int l, uint8_t* state) {
   const int64_t nx = nx_at(g, l), n = nx * ny_at(g, l);
   // block size at this level: 8 * extent / (max(bpdx, bpdy) * 8 * 2^l), as forest.cpp cell_h
   const double h = __ddiv_rn(g.extent, __dmul_rn(__dmul_rn((double)max(g.bpdx, g.bpdy), 8.0), (double)(1ll << l)));
   const double bs = __dmul_rn(8.0, h);
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t p = grid_thread(); p < n; p += grid_threads()) {
     const int64_t i = p % nx, j = p / nx;
     bool exists = l == 0;
-    if (!exists) exists = state[g.off[l - 1] + (j >> 1) * nx_at(g, l - 1) + (i >> 1)] == kRefined;
+    if (!exists) exists = __ldcg(state + g.off[l - 1] + (j >> 1) * nx_at(g, l - 1) + (i >> 1)) == kRefined;
     uint8_t st = kAbsent;
     if (exists) {
       bool refine = false;
@@ -84,18 +96,17 @@ __global__ void k_adapt_tag(const __grid_constant__ AdaptGeom g, const __grid_co
 __device__ __forceinline__ int covering_level(const AdaptGeom& g, const uint8_t* state, int l, int64_t i, int64_t j) {
   for (int q = l; q >= 0; --q) {
     const int sh = l - q;
-    const uint8_t s = state[g.off[q] + (j >> sh) * nx_at(g, q) + (i >> sh)];
+    const uint8_t s = __ldcg(state + g.off[q] + (j >> sh) * nx_at(g, q) + (i >> sh));
     if (s == kLeaf || s == kSplit) return q;
     if (s == kRefined) return -1;
   }
   return -1;
 }
 
-__global__ void k_adapt_mark(const __grid_constant__ AdaptGeom g, int l, uint8_t* __restrict__ state,
-                             int* __restrict__ changed) {
+__device__ __forceinline__ void adapt_mark(const AdaptGeom& g, int l, uint8_t* state, int* changed) {
   const int64_t nx = nx_at(g, l), ny = ny_at(g, l), n = nx * ny;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    const uint8_t s = state[g.off[l] + p];
+  for (int64_t p = grid_thread(); p < n; p += grid_threads()) {
+    const uint8_t s = __ldcg(state + g.off[l] + p);
     if (s != kLeaf && s != kSplit) continue;
     const int64_t i = p % nx, j = p / nx;
     for (int dj = -1; dj <= 1; ++dj)
@@ -121,10 +132,10 @@ __global__ void k_adapt_mark(const __grid_constant__ AdaptGeom g, int l, uint8_t
 }
 
 // Splits the marked leaves of level l into their four children.
-__global__ void k_adapt_split(const __grid_constant__ AdaptGeom g, int l, uint8_t* __restrict__ state) {
+__device__ __forceinline__ void adapt_split(const AdaptGeom& g, int l, uint8_t* state) {
   const int64_t nx = nx_at(g, l), n = nx * ny_at(g, l);
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    if (state[g.off[l] + p] != kSplit) continue;
+  for (int64_t p = grid_thread(); p < n; p += grid_threads()) {
+    if (__ldcg(state + g.off[l] + p) != kSplit) continue;
     state[g.off[l] + p] = kRefined;
     const int64_t i = p % nx, j = p / nx, cnx = nx_at(g, l + 1);
     for (int c = 0; c < 4; ++c)
@@ -148,34 +159,107 @@ __device__ __forceinline__ uint64_t leaf_key(const AdaptGeom& g, int l, int64_t 
 }
 
 // mark[key] = 1 for every leaf (the array is cleared before)
-__global__ void k_adapt_keys(const __grid_constant__ AdaptGeom g, int l, const uint8_t* __restrict__ state,
-                             int32_t* __restrict__ mark) {
+__device__ __forceinline__ void adapt_keys(const AdaptGeom& g, int l, const uint8_t* state, int32_t* mark) {
   const int64_t nx = nx_at(g, l), n = nx * ny_at(g, l);
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
-    if (state[g.off[l] + p] == kLeaf) mark[leaf_key(g, l, p % nx, p / nx)] = 1;
+  for (int64_t p = grid_thread(); p < n; p += grid_threads())
+    if (__ldcg(state + g.off[l] + p) == kLeaf) mark[leaf_key(g, l, p % nx, p / nx)] = 1;
 }
 
-__global__ void k_adapt_scatter(const __grid_constant__ AdaptGeom g, int l, const uint8_t* __restrict__ state,
-                                const int32_t* __restrict__ rank, int64_t nb, int32_t* __restrict__ level,
-                                int32_t* __restrict__ bx, int32_t* __restrict__ by, int* __restrict__ err) {
-  const int64_t nx = nx_at(g, l), n = nx * ny_at(g, l);
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
-    if (state[g.off[l] + p] == kLeaf) {
-      const int64_t i = p % nx, j = p / nx;
-      const int32_t b = rank[leaf_key(g, l, i, j)];
-      if (b < 0 || b >= nb) {  // cannot happen for a consistent scan; never write outside the arrays
-        atomicExch(err, 1);
-        continue;
-      }
-      level[b] = l;
-      bx[b] = (int32_t)i;
-      by[b] = (int32_t)j;
+// rank[i] = marks before i over the dense key array, and their total: each CTA
+// counts its share of the keys, and after the barrier every CTA adds the counts
+// before its own.  Returns false if the barrier gave up.
+__device__ __forceinline__ bool adapt_rank(Team& team, const int32_t* mark, int64_t K, int32_t* rank, int32_t* sums,
+                                           int32_t* total) {
+  __shared__ int warp_base[kAdaptThreads / 32];
+  __shared__ int before;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t k0 = K * (int64_t)blockIdx.x / gridDim.x, k1 = K * (int64_t)(blockIdx.x + 1) / gridDim.x;
+  int count = 0;
+  for (int64_t t = k0; t < k1; t += kAdaptThreads) {
+    const int64_t i = t + threadIdx.x;
+    count += __syncthreads_count(i < k1 && __ldcg(mark + i) != 0);
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = count;
+  if (!team.sync(0)) return false;
+  if (w == 0) {
+    int a = 0;
+    for (int c = lane; c < (int)blockIdx.x; c += 32) a += __ldcg(sums + c);
+    a = warp_sum(a);
+    if (lane == 0) before = a;
+  }
+  __syncthreads();
+  int base = before;
+  for (int64_t t = k0; t < k1; t += kAdaptThreads) {
+    const int64_t i = t + threadIdx.x;
+    const unsigned m = __ballot_sync(kFull, i < k1 && __ldcg(mark + i) != 0);
+    if (lane == 0) warp_base[w] = __popc(m);
+    __syncthreads();
+    int b = base, all = 0;
+    for (int q = 0; q < kAdaptThreads / 32; ++q) {
+      if (q < w) b += warp_base[q];
+      all += warp_base[q];
     }
+    if (i < k1) rank[i] = b + __popc(m & ((1u << lane) - 1u));
+    base += all;
+    __syncthreads();
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = base;
+  return true;
 }
 
-unsigned grid_for(int64_t n) {
-  const int64_t b = (n + 255) / 256;
-  return (unsigned)(b < 4096 ? (b > 0 ? b : 1) : 4096);
+__global__ void __launch_bounds__(kAdaptThreads, 1)
+    k_adapt_build(const __grid_constant__ AdaptGeom g, const __grid_constant__ AdaptDisks D,
+                  const __grid_constant__ AdaptScratch sc, int64_t K, unsigned long long timeout_ns) {
+  __shared__ Team team;
+  AdaptFlags& F = *sc.flags;
+  if (threadIdx.x == 0) team.init(blockIdx.x, gridDim.x, &F.counter, nullptr, &F.abort_flag, timeout_ns, nullptr);
+  __syncthreads();
+  for (int64_t i = grid_thread(); i < K; i += grid_threads()) sc.mark[i] = 0;
+  for (int l = 0; l < g.L; ++l) {
+    adapt_tag(g, D, l, sc.state);
+    if (!team.sync(0)) return;
+  }
+  // balance: rounds of descending levels until one marks nothing.  A round
+  // carries the splits it causes down to the coarse levels, so two rounds
+  // settle it in practice; the bound only guards the loop.
+  bool settled = false;
+  for (int round = 0; round < 4 * g.L + 4 && !settled; ++round) {
+    for (int l = g.L - 1; l >= 2; --l) {
+      adapt_mark(g, l, sc.state, &F.changed[round]);
+      if (!team.sync(0)) return;
+      // the marked leaves of every coarser level: their children are leaves,
+      // not marked ones, so the levels do not affect each other
+      for (int q = l - 2; q >= 0; --q) adapt_split(g, q, sc.state);
+      if (!team.sync(0)) return;
+    }
+    settled = __ldcg(&F.changed[round]) == 0;  // written before the last barrier: the same for all
+  }
+  if (!settled) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) F.unsettled = 1;
+    return;
+  }
+  for (int l = 0; l < g.L; ++l) adapt_keys(g, l, sc.state, sc.mark);
+  if (!team.sync(0)) return;
+  adapt_rank(team, sc.mark, K, sc.rank, sc.sums, &F.leaves);
+}
+
+__global__ void k_adapt_scatter(const __grid_constant__ AdaptGeom g, const __grid_constant__ AdaptScratch sc, int64_t nb,
+                                int32_t* __restrict__ level, int32_t* __restrict__ bx, int32_t* __restrict__ by) {
+  for (int l = 0; l < g.L; ++l) {
+    const int64_t nx = nx_at(g, l), n = nx * ny_at(g, l);
+    for (int64_t p = grid_thread(); p < n; p += grid_threads())
+      if (sc.state[g.off[l] + p] == kLeaf) {
+        const int64_t i = p % nx, j = p / nx;
+        const int32_t b = sc.rank[leaf_key(g, l, i, j)];
+        if (b < 0 || b >= nb) {  // cannot happen for a consistent scan; never write outside the arrays
+          atomicExch(&sc.flags->scatter_err, 1);
+          continue;
+        }
+        level[b] = l;
+        bx[b] = (int32_t)i;
+        by[b] = (int32_t)j;
+      }
+  }
 }
 
 }  // namespace
@@ -189,50 +273,40 @@ int64_t adapt_key_space(int bpdx, int bpdy, int level_max) {
 
 int adapt_build(const AdaptGeom& g, const AdaptDisks& D, const AdaptScratch& sc, int64_t* nleaves,
                 cudaStream_t s) {
-  for (int l = 0; l < g.L; ++l)
-    k_adapt_tag<<<grid_for(((int64_t)g.bpdx << l) * ((int64_t)g.bpdy << l)), 256, 0, s>>>(g, D, l, sc.state);
-  // balance: rounds of descending levels until one marks nothing.  A round
-  // carries the splits it causes down to the coarse levels, so two rounds
-  // settle it in practice; the bound only guards the loop.
-  bool settled = false;
-  for (int round = 0; round < 4 * g.L + 4 && !settled; ++round) {
-    if (cudaMemsetAsync(sc.changed, 0, sizeof(int), s) != cudaSuccess) return CUP2D_CUDA_ERROR;
-    for (int l = g.L - 1; l >= 2; --l) {
-      const int64_t n = ((int64_t)g.bpdx << l) * ((int64_t)g.bpdy << l);
-      k_adapt_mark<<<grid_for(n), 256, 0, s>>>(g, l, sc.state, sc.changed);
-      for (int q = l - 2; q >= 0; --q)
-        k_adapt_split<<<grid_for(((int64_t)g.bpdx << q) * ((int64_t)g.bpdy << q)), 256, 0, s>>>(g, q, sc.state);
-    }
-    int changed = 0;
-    if (cudaMemcpyAsync(&changed, sc.changed, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-      return CUP2D_CUDA_ERROR;
-    settled = changed == 0;
-  }
-  if (!settled) return CUP2D_BAD_MESH;
-  const int64_t K = adapt_key_space(g.bpdx, g.bpdy, g.L);
-  if (cudaMemsetAsync(sc.mark, 0, sizeof(int32_t) * K, s) != cudaSuccess) return CUP2D_CUDA_ERROR;
-  for (int l = 0; l < g.L; ++l)
-    k_adapt_keys<<<grid_for(((int64_t)g.bpdx << l) * ((int64_t)g.bpdy << l)), 256, 0, s>>>(g, l, sc.state, sc.mark);
-  // rank[0..K) exclusive prefix of the marks, rank[K] their total: the leaf count
-  if (launch_exclusive_scan(sc.mark, K, sc.rank, sc.scan_tmp, s) != cudaSuccess) return CUP2D_CUDA_ERROR;
-  int32_t count = 0;
-  if (cudaMemcpyAsync(&count, sc.rank + K, sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return CUP2D_CUDA_ERROR;
-  *nleaves = count;
-  return cudaGetLastError() == cudaSuccess ? CUP2D_OK : CUP2D_CUDA_ERROR;
+  const int64_t finest = ((int64_t)g.bpdx << (g.L - 1)) * ((int64_t)g.bpdy << (g.L - 1));
+  const int grid =
+      (int)std::max<int64_t>(1, std::min<int64_t>({(finest + kAdaptThreads - 1) / kAdaptThreads, sms, kAdaptMaxCtas}));
+  int64_t K = adapt_key_space(g.bpdx, g.bpdy, g.L);
+  unsigned long long timeout_ns = 20000000000ull;
+  void* args[] = {const_cast<AdaptGeom*>(&g), const_cast<AdaptDisks*>(&D), const_cast<AdaptScratch*>(&sc), &K,
+                  &timeout_ns};
+  AdaptFlags f;
+  if (cudaMemsetAsync(sc.flags, 0, sizeof(AdaptFlags), s) != cudaSuccess ||
+      cudaLaunchCooperativeKernel((const void*)k_adapt_build, dim3(grid), dim3(kAdaptThreads), args, 0, s) !=
+          cudaSuccess ||
+      cudaMemcpyAsync(&f, sc.flags, sizeof(AdaptFlags), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
+    cudaGetLastError();
+    return CUP2D_CUDA_ERROR;
+  }
+  if (f.abort_flag) return CUP2D_TIMEOUT;
+  if (f.unsettled) return CUP2D_BAD_MESH;
+  *nleaves = f.leaves;
+  return CUP2D_OK;
 }
 
 int adapt_scatter(const AdaptGeom& g, const AdaptScratch& sc, int64_t nb, int32_t* level, int32_t* bx, int32_t* by,
                   cudaStream_t s) {
-  if (cudaMemsetAsync(sc.changed, 0, sizeof(int), s) != cudaSuccess) return CUP2D_CUDA_ERROR;
-  for (int l = 0; l < g.L; ++l)
-    k_adapt_scatter<<<grid_for(((int64_t)g.bpdx << l) * ((int64_t)g.bpdy << l)), 256, 0, s>>>(
-        g, l, sc.state, sc.rank, nb, level, bx, by, sc.changed);
+  const int64_t finest = ((int64_t)g.bpdx << (g.L - 1)) * ((int64_t)g.bpdy << (g.L - 1));
+  k_adapt_scatter<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((finest + 255) / 256, 4096)), 256, 0, s>>>(
+      g, sc, nb, level, bx, by);
   int err = 0;
   if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(&err, sc.changed, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaMemcpyAsync(&err, &sc.flags->scatter_err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return CUP2D_CUDA_ERROR;
   return err ? CUP2D_BAD_MESH : CUP2D_OK;

@@ -221,12 +221,17 @@ __global__ void k_classify(ForestDev F, int32_t* __restrict__ nbr, unsigned long
   hblk[b] = h0 / (double)(1ll << l);
 }
 
-// The leaf at the domain's (0, 0) corner: the block whose index is (0, 0) at
-// its level (ExpAMRSolver.cpp:251-256 places bMeanConstraint's row there).
-__global__ void k_origin(ForestDev F, int* __restrict__ out) {
+// What the host needs of an assembly, in one place for one read-back: err[0]
+// the error flag (set before), then the leaf at the domain's (0, 0) corner (the
+// block whose index is (0, 0) at its level: ExpAMRSolver.cpp:251-256 places
+// bMeanConstraint's row there), the explicit rows and their entries.
+__global__ void k_collect(ForestDev F, const int32_t* __restrict__ rows, const int32_t* __restrict__ nnz,
+                          int* __restrict__ err) {
   int32_t b = -1;
   for (int l = 0; l < F.L && b < 0; ++l) b = F.leaf(l, 0, 0);
-  *out = b;
+  err[1] = b;
+  err[2] = *rows;
+  err[3] = *nnz;
 }
 
 // ------------------------------------------------------------- scans ------
@@ -543,7 +548,6 @@ int assemble_on_device(const AssembleIn& in, DeviceMesh& out, cudaStream_t s) {
   if (cudaMemsetAsync(out.err, 0, sizeof(int), s) != cudaSuccess) return CUP2D_CUDA_ERROR;
   k_fill_tables<<<g, 256, 0, s>>>(F, out.table, out.err);
   k_classify<<<g, 256, 0, s>>>(F, out.nbr, out.xmask, out.xcount, out.hblk, in.h0, out.err);
-  k_origin<<<1, 1, 0, s>>>(F, out.err + 1);
   launch_exclusive_scan(out.xcount, nb, out.xbase, out.scan_tmp, s);
   // Row arrays at their bound (a block's explicit rows are cells of its four
   // faces: at most 28), so that the row lengths are built and scanned before
@@ -556,14 +560,13 @@ int assemble_on_device(const AssembleIn& in, DeviceMesh& out, cudaStream_t s) {
   k_rows<<<(unsigned)nb, 64, 0, s>>>(F, out.xmask, out.xbase, out.rowlen, out.rowcell, nullptr, nullptr, nullptr, 0,
                                      cap, out.err);
   launch_exclusive_scan(out.rowlen, cap, out.xptr, out.scan_tmp, s);
+  k_collect<<<1, 1, 0, s>>>(F, out.xbase + nb, out.xptr + cap, out.err);
   if (cudaGetLastError() != cudaSuccess) return CUP2D_CUDA_ERROR;
-  int32_t hR = 0, hnnz = 0;
-  int herr[2] = {0, -1};
-  if (cudaMemcpyAsync(&hR, out.xbase + nb, sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaMemcpyAsync(&hnnz, out.xptr + cap, sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaMemcpyAsync(herr, out.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  int herr[kAssembleFlags] = {0, -1, 0, 0};
+  if (cudaMemcpyAsync(herr, out.err, sizeof(herr), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return CUP2D_CUDA_ERROR;
+  const int32_t hR = herr[2], hnnz = herr[3];
   if (herr[0] != 0 || herr[1] < 0 || hR > cap) return CUP2D_BAD_MESH;
   out.origin = herr[1];
   out.R = hR;

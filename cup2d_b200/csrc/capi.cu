@@ -187,7 +187,8 @@ struct cup2d_poisson {
   // device forest adaptation: per-level states, Morton key marks and ranks,
   // scan scratch, flag
   DevBuf<uint8_t> ad_state;
-  DevBuf<int32_t> ad_mark, ad_rank, ad_scan, ad_flags;
+  DevBuf<int32_t> ad_mark, ad_rank, ad_sums;
+  DevBuf<AdaptFlags> ad_flags;
   DevBuf<double> ps_part;  // pressure step: weighted-mean partials
   uint64_t mesh_version = 0;
   bool profiling = false;
@@ -263,7 +264,7 @@ int assemble_blocks(cup2d_poisson* h, const cup2d_forest* f, int64_t nb) {
   const int64_t entries = leaf_table_entries(f->bpdx, f->bpdy, f->level_max);
   if ((st = h->table.ensure(entries)) || (st = h->nbr.ensure(4 * nb)) || (st = h->xmask.ensure(nb)) ||
       (st = h->xcount.ensure(nb)) || (st = h->xbase.ensure(nb + 1)) || (st = h->hblk.ensure(nb)) ||
-      (st = h->scan_tmp.ensure(scan_temp_ints(n) + 2)) || (st = h->err.ensure(2)))
+      (st = h->scan_tmp.ensure(scan_temp_ints(n) + 2)) || (st = h->err.ensure(kAssembleFlags)))
     return st;
   // the best-iterate copy; the Krylov vectors of a precision are allocated
   // by its first solve
@@ -518,10 +519,10 @@ int cup2d_poisson_adapt_disks(cup2d_poisson* h, int32_t ndisks, const double* di
   // buffers may be reallocated: let solves queued on any stream finish first
   if (cudaDeviceSynchronize() != cudaSuccess) return CUP2D_CUDA_ERROR;
   int st;
-  if ((st = h->ad_state.ensure(off)) || (st = h->ad_mark.ensure(K)) || (st = h->ad_rank.ensure(K + 1)) ||
-      (st = h->ad_scan.ensure(scan_temp_ints(K) + 2)) || (st = h->ad_flags.ensure(1)))
+  if ((st = h->ad_state.ensure(off)) || (st = h->ad_mark.ensure(K)) || (st = h->ad_rank.ensure(K)) ||
+      (st = h->ad_sums.ensure(kAdaptMaxCtas)) || (st = h->ad_flags.ensure(1)))
     return st;
-  const AdaptScratch sc{h->ad_state.p, h->ad_mark.p, h->ad_rank.p, h->ad_scan.p, h->ad_flags.p};
+  const AdaptScratch sc{h->ad_state.p, h->ad_mark.p, h->ad_rank.p, h->ad_sums.p, h->ad_flags.p};
   int64_t nb = 0;
   if ((st = adapt_build(g, D, sc, &nb, h->stream))) return st;
   if (nb <= 0 || nb > (int64_t)(INT32_MAX / kBLEN)) return CUP2D_BAD_MESH;

@@ -34,7 +34,7 @@ struct DeviceMesh {
   int32_t* xbase = nullptr;       // [nb+1]
   double* hblk = nullptr;         // [nb]
   int32_t* scan_tmp = nullptr;
-  int* err = nullptr;             // [2]: error flag, then the origin block
+  int* err = nullptr;             // [kAssembleFlags]: error flag, origin block, explicit rows, their entries
   int32_t origin = -1;            // leaf at the domain's (0, 0) corner (read back)
   int64_t R = 0, nnz = 0;
   int32_t* rowlen = nullptr;      // [R]
@@ -64,6 +64,7 @@ struct DeviceMesh {
   }
 };
 
+constexpr int kAssembleFlags = 4;
 // Explicit (coarse/fine) rows of one block at most: the cells on its four faces.
 constexpr int64_t kMaxExplicitRowsPerBlock = 28;
 
@@ -251,18 +252,29 @@ struct AdaptDisks {
   double band;
   double d[kMaxAdaptDisks][3];  // cx, cy, r
 };
+// Launch state and results, zeroed before a build.
+struct AdaptFlags {
+  unsigned counter;   // grid barrier
+  int abort_flag;
+  int leaves;         // their number
+  int unsettled;      // the balance did not settle
+  int scatter_err;
+  int changed[4 * kMaxLevels + 4];  // per balance round
+};
+constexpr int kAdaptMaxCtas = 1024;
 struct AdaptScratch {
   uint8_t* state;    // [leaf_table_entries]
   int32_t* mark;     // [adapt_key_space]
-  int32_t* rank;     // [adapt_key_space + 1]: exclusive prefix sums, then the total
-  int32_t* scan_tmp; // [scan_temp_ints(adapt_key_space)]
-  int* changed;      // [1]: balance round flag, scatter error flag
+  int32_t* rank;     // [adapt_key_space]: exclusive prefix sums of the marks
+  int32_t* sums;     // [kAdaptMaxCtas]
+  AdaptFlags* flags;
 };
 // Size of the dense Morton key space of a forest's leaves (a power of 4).
 int64_t adapt_key_space(int bpdx, int bpdy, int level_max);
 // Tags, balances and orders the leaves; returns their number in *nleaves
 // (read back: the caller sizes the block arrays with it).  CUP2D_OK,
-// CUP2D_CUDA_ERROR, or CUP2D_BAD_MESH if the balance did not settle.
+// CUP2D_CUDA_ERROR, CUP2D_TIMEOUT, or CUP2D_BAD_MESH if the balance did not
+// settle.
 int adapt_build(const AdaptGeom& g, const AdaptDisks& D, const AdaptScratch& sc, int64_t* nleaves,
                 cudaStream_t s);
 // Writes the nb leaves (level, bx, by) in Morton order (CUP2D_OK, or an error

@@ -98,3 +98,19 @@ def test_adapt_arguments(cuda):
         assert s.ncells == m.ncells
         x = s.solve(m.rhs_fourier(1))
         assert s.last_stats["status"] == L.OK and x.shape == (m.ncells,)
+
+
+@pytest.mark.parametrize("bpdx,bpdy,levels", [(1, 1, 1), (3, 5, 1), (7, 3, 2), (1, 1, 6), (33, 17, 3)])
+def test_device_forest_root_grids(cuda, bpdx, bpdy, levels):
+    """Forests at the edges of the one-launch build: one level (nothing to
+    balance), fewer positions than a CTA has threads, root grids that are no
+    power of two (keys without a leaf), key ranges of several tiles a CTA."""
+    ext = 1.0
+    disks = [(0.4 * ext, 0.3 * ext * bpdy / max(bpdx, bpdy), 0.1)]
+    host = Mesh.disks(bpdx, bpdy, levels, ext, disks, 0.03)
+    with Solver(Mesh.uniform(bpdx, bpdy, levels, 0, ext)) as s:
+        dev = s.adapt_disks(disks, 0.03)
+        again = s.adapt_disks(disks, 0.03)
+    for m in (dev, again):
+        assert np.array_equal(m.level, host.level)
+        assert np.array_equal(m.bx, host.bx) and np.array_equal(m.by, host.by)
