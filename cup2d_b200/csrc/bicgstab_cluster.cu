@@ -11,7 +11,7 @@
 // (a cluster barrier's acquire drops L1, so tables left in global memory cost
 // two dependent L2 reads in every SpMV).  Barriers are the cluster's hardware
 // barrier, and a reduction posts each CTA's partial into every CTA's shared
-// memory before it.
+// memory.
 //
 // The iteration, its scalars and its stop tests are those of the grid solver,
 // with one rearrangement: the solution update x += alpha z + omega z2 is kept
@@ -20,18 +20,17 @@
 // true-residual replacement (mixed).  So z and z2 share one buffer and neither
 // is read again after its SpMV.  y is FP64 in both forms.
 //
-// Solves, against the grid solver: 128 blocks FP64 2.01 -> 0.81 ms (100
-// iterations), 302 blocks through the host interface 4.1 -> 1.8 ms.  What is left
-// of an iteration at 128 blocks (7.3 us, 14k clocks): 4.8k in the two SpMV passes
-// (dependent shared loads), 6.3k in the three reductions (the cluster barrier
-// alone takes 480 clocks, 1020 behind remote stores), 2.4k in the block solves.
+// us an iteration, against the grid solver: FP64 128 blocks 18.5 -> 6.7, 449 17.9 ->
+// 9.2; mixed 128 19.0 -> 8.7, 1,502 19.8 -> 16.9.  What is left of one at 128 blocks
+// (13k clocks): 4.8k in the two SpMV passes (dependent shared loads), some 4.5k in
+// the three reductions, 2.4k in the block solves, 1.2k in the two barriers.
 //
 // Copies of the neighbours' blocks pushed ahead of each SpMV, so that no load
 // left the CTA, measured no faster (their stores cost what the loads had).
 //
-// The waits end by construction: the CTAs of a cluster are co-resident and
-// pass the same barriers; the deadline is one of pass E's reduced quantities,
-// so all CTAs leave together.
+// The CTAs of a cluster are co-resident and pass the same barriers; the
+// deadline is one of pass E's reduced quantities, so all CTAs leave together.
+// The polls of a reduction are bounded besides.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -50,6 +49,7 @@ constexpr int kClThreads = 512;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kMaxCluster = 16;
 constexpr int kMaxSweep = 64;  // mixed: longest FP32 sweep between true residuals
+constexpr unsigned kMaxPolls = 1u << 23;  // bound of a reduction's wait, some 0.3 s
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, unsigned rank) {
   uint32_t a;
@@ -96,8 +96,14 @@ __device__ __forceinline__ void ld_cluster2_if(bool p, uint32_t a, float (&v)[2]
                : "r"(a), "r"((unsigned)p));
 }
 constexpr uint32_t kCodes = 1u;  // neighbour entries up to here: 0 wall, 1 coarse/fine face
-__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+// Two 64-bit words; each is written and read whole.
+__device__ __forceinline__ void st_cluster_words(uint32_t a, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_words(uint32_t a) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
+  return v;
 }
 __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
@@ -112,9 +118,12 @@ __device__ __forceinline__ double prod(float a, float b) { return (double)a * (d
 struct ClHead {
   double wred[kClWarps][kRedMax];
   double out[2][kRedMax];                // the last two reductions' results
-  double post[2][kRedMax][kMaxCluster];  // the CTAs' partials, posted by each into every CTA
+  // the CTAs' partials, posted by each into every CTA: {tag, low half} and
+  // {tag, high half} of a double
+  alignas(16) ulonglong2 post[2][kRedMax][kMaxCluster];
   double sine[32][4];                    // mixed: the FP64 block solve's constants per lane
   unsigned nlong;                        // explicit rows longer than kRowWidth
+  int lost;                              // a partial did not arrive
 };
 
 constexpr int kSlotBytes = 512;  // one chunk of one vector: 16 bytes a lane
@@ -220,26 +229,39 @@ struct Cluster {
   unsigned posts;
 
   // Sums (bit q of is_max: maxima) of v over the cluster's threads, in out.
-  // A full barrier: what any thread wrote before it is visible after it.
+  // Each CTA writes its partial, tagged, into every CTA's shared memory and
+  // waits for the others' in its own: one way across (a cluster barrier behind
+  // the same stores took 740 clocks on 8 CTAs and 1020 on 16).  A CTA posts
+  // after all its warps have finished the pass, so what follows may overwrite
+  // what the pass read; it orders no other data (that takes cluster_sync).
+  // The wait is bounded: past it head.lost is set, and the caller leaves.
   template <int NV>
-  __device__ __forceinline__ void reduce(const double (&v)[NV], unsigned is_max, double (&out)[NV]) {
+  __device__ __forceinline__ bool reduce(const double (&v)[NV], unsigned is_max, double (&out)[NV]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     warp_partials<NV>(v, is_max, head.wred[w]);
     __syncthreads();
-    const unsigned set = ++posts & 1u;
-    const bool mx = (is_max >> w) & 1u;
+    const unsigned tag = ++posts, set = tag & 1u;
     if (w < NV) {
+      const bool mx = (is_max >> w) & 1u;
       double r = head.wred[lane & (kClWarps - 1)][w];
 #pragma unroll
       for (int o = kClWarps / 2; o > 0; o >>= 1) {
         const double b = __shfl_xor_sync(kFull, r, o);
         r = mx ? nanmax(r, b) : r + b;
       }
-      if (lane < (int)size) st_cluster(cluster_addr(smem_u32(&head.post[set][w][rank]), (unsigned)lane), r);
-    }
-    cluster_sync();
-    if (w < NV) {
-      double r = lane < (int)size ? head.post[set][w][lane] : 0.0;
+      const unsigned long long t = (unsigned long long)tag << 32;
+      if (lane < (int)size)
+        st_cluster_words(cluster_addr(smem_u32(&head.post[set][w][rank]), (unsigned)lane),
+                         t | (unsigned)__double2loint(r), t | (unsigned)__double2hiint(r));
+      ulonglong2 x = make_ulonglong2(0ull, 0ull);
+      unsigned spins = 0;
+      bool ready;
+      do {
+        if (lane < (int)size) x = ld_words(smem_u32(&head.post[set][w][lane]));
+        ready = lane >= (int)size || ((unsigned)(x.x >> 32) == tag && (unsigned)(x.y >> 32) == tag);
+      } while (!__all_sync(kFull, ready) && ++spins < kMaxPolls);
+      if (spins >= kMaxPolls && lane == 0) head.lost = 1;
+      r = lane < (int)size ? __hiloint2double((int)(unsigned)x.y, (int)(unsigned)x.x) : 0.0;
 #pragma unroll
       for (int o = kMaxCluster / 2; o > 0; o >>= 1) {
         const double b = __shfl_xor_sync(kFull, r, o);
@@ -250,6 +272,7 @@ struct Cluster {
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NV; ++q) out[q] = head.out[set][q];
+    return head.lost == 0;
   }
 
   __device__ __forceinline__ void st_z(int c, int lane, const T (&v)[N]) const {
@@ -508,7 +531,12 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
       const unsigned k = (unsigned)(((long long)(b + 1) * size - 1) / nb);
       addr[b] = cluster_addr(zbase + (uint32_t)((b - share(nb, k, size)) * kBLEN * sizeof(T)), k);
     }
-    if (threadIdx.x == 0) head.nlong = 0u;
+    if (threadIdx.x == 0) {
+      head.nlong = 0u;
+      head.lost = 0;
+    }
+    for (int i = threadIdx.x; i < 2 * kRedMax * kMaxCluster; i += kClThreads)
+      (&head.post[0][0][0])[i] = make_ulonglong2(0ull, 0ull);  // no tag
     if (MIXED && w == 0) {
       SineSolve<double> d;
       d.init();
@@ -568,18 +596,19 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
   };
   double* const row = reinterpret_cast<double*>(C.scratch);
   double mean_b = 0.0;
+  bool lost = false;  // a reduction gave up: the same for the CTA, which then leaves
   if constexpr (MIXED) {  // Neumann compatibility: project b to zero sum
     double v[1] = {0.0}, o[1];
     for (int blk = b0 + w; blk < b1; blk += kClWarps)
       v[0] += __ldg(V.b + blk * kBLEN + lane) + __ldg(V.b + blk * kBLEN + lane + 32);
-    C.reduce(v, 0u, o);
+    lost = !C.reduce(v, 0u, o);
     mean_b = o[0] / (double)(M.nb * kBLEN);
   }
   // r = b - A x (BiCGSTAB.cu:430-465)
   auto residual = [&](bool set_rh, double (&o)[6]) {
     ClResidual<T> epi{K, V.b, mean_b, set_rh, {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}};
     spmv_range<double>(M, V.x, b0, b1, C.r0, C.r1, epi, row);
-    C.reduce(epi.v, 0x23u, o);
+    lost = !C.reduce(epi.v, 0x23u, o) || lost;
   };
   double q[6];
   residual(true, q);
@@ -642,7 +671,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
         C.spmv(epi);
         const double v[1] = {epi.acc};
         double o[1];
-        C.reduce(v, 0u, o);
+        lost = !C.reduce(v, 0u, o) || lost;
         alpha = rho / (o[0] + eps);
       }
       // pass C: s = r - alpha nu (in place of r); z = P^-1 s
@@ -666,7 +695,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
         C.spmv(epi);
         const double v[2] = {epi.ts, epi.tt};
         double o[2];
-        C.reduce(v, 0u, o);
+        lost = !C.reduce(v, 0u, o) || lost;
         omega = o[0] / (o[1] + eps);
       }
       // pass E: y += alpha p, y += omega s; r = s - omega t; norms; the
@@ -710,9 +739,9 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
                 make_double2(yv[2 * j], yv[2 * j + 1]);
         }
         if (threadIdx.x == 0 && globaltimer_ns() > deadline) v[4] = 1.0;
-        C.reduce(v, 0x11u, e);
+        lost = !C.reduce(v, 0x11u, e) || lost;
       }
-      if (e[4] != 0.0) {
+      if (e[4] != 0.0 || lost) {
         expired = true;
         break;
       }
@@ -776,8 +805,8 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
       }
     }
   }
-  if (expired) {  // the same in every CTA
-    if (rank == 0 && threadIdx.x == 0) atomicExch(S.abort_flag, 1);
+  if (expired || lost) {  // the deadline: the same in every CTA
+    if (threadIdx.x == 0) atomicExch(S.abort_flag, 1);
     cluster_sync();
     return;
   }
@@ -805,7 +834,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
     hx[1] += 2.0 * (h * h);
   }
   double o[2] = {0.0, 1.0};
-  if (sp.subtract_mean) C.reduce(hx, 0u, o);
+  if (sp.subtract_mean && !C.reduce(hx, 0u, o) && threadIdx.x == 0) atomicExch(S.abort_flag, 1);
   const double avg = sp.subtract_mean ? o[0] / o[1] : 0.0;
   for (int lb = w; lb < nbl; lb += kClWarps) {
     double xv[2];
@@ -883,12 +912,11 @@ size_t cluster_limit(int device) {
 }  // namespace
 
 // The cluster solver takes every forest whose vectors fit (FP64 about 940
-// blocks, mixed 1,650): us an iteration against the grid solver, FP64 128
-// blocks 7.3 / 18.5, 449 10.1 / 17.9, 929 16.5 / 19.1; mixed 128 9.4 / 19.0, 449
-// 10.3 / 18.1, 1,502 17.9 / 19.8.  Of the cluster sizes the smallest with at
-// most 12 blocks a CTA: FP64 65 blocks 9.7 / 7.7 / 6.2 / 6.6 us on 2 / 4 / 8 / 16
-// CTAs (the barrier grows with the cluster), 128 blocks 9.8 / 7.6 / 7.3 on 4 / 8
-// / 16, 302 blocks 11.7 / 9.6 on 8 / 16.
+// blocks, mixed 1,650), where it is still the faster one: us an iteration
+// against the grid solver, FP64 929 blocks 14.9 / 17.8, mixed 1,502 16.9 / 19.6.  Of
+// the cluster sizes the smallest with at most 12 blocks a CTA (with barriers in
+// place of the tagged reductions: FP64 65 blocks 9.7 / 7.7 / 6.2 / 6.6 us on 2 / 4 /
+// 8 / 16 CTAs, 128 blocks 9.8 / 7.6 / 7.3 on 4 / 8 / 16, 302 blocks 11.7 / 9.6 on 8 / 16).
 template <class T>
 int cluster_size(int device, int64_t nb) {
   const size_t most = cluster_limit(device);
