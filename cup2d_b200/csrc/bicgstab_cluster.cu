@@ -333,7 +333,8 @@ struct Cluster {
       epi.chunk(c, lane, out, skip);
     }
     const T* __restrict__ vals = row_vals<T>(M);
-    for (int i = (int)threadIdx.x; i < r1 - r0; i += kClThreads) {
+    // from the last warp down: the first ones have one chunk more, or the only one
+    for (int i = kClThreads - 1 - (int)threadIdx.x; i < r1 - r0; i += kClThreads) {
       T acc = T(0);
       int cell, k, k1;  // entries [k, k1) are left to the tables in global memory
       if (i < kept) {
