@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -154,6 +155,14 @@ int from_cuda(cudaError_t e) {
 
 }  // namespace
 
+// Launch state and results of a single solve: the first two words are zeroed
+// before the launch, the whole is read back in one copy after it.
+struct SolveCtl {
+  unsigned bar;      // arrival counter of the grid barrier
+  int abort_flag;
+  DevStats stats;
+};
+
 struct cup2d_poisson {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -179,9 +188,7 @@ struct cup2d_poisson {
   DevBuf<float> f_r, f_rh, f_p, f_nu, f_t, f_z, f_z2;
   // persistent-kernel scratch
   DevBuf<double> red;
-  DevBuf<unsigned> bar;
-  DevBuf<int> abort_flag;
-  DevBuf<DevStats> dstats;
+  DevBuf<SolveCtl> ctl;
   DevBuf<unsigned long long> prof;  // phase timers (profiling on)
   DevBuf<double> rhs_coef, rhs_part;  // device RHS: coefficients, partial sums + mean
   // device forest adaptation: per-level states, Morton key marks and ranks,
@@ -193,7 +200,7 @@ struct cup2d_poisson {
   uint64_t mesh_version = 0;
   bool profiling = false;
   int prof_grid = 0;                // grid of the profiled solves
-  DevStats* hstats = nullptr;  // pinned
+  SolveCtl* hctl = nullptr;  // pinned
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int grid64 = 0, gridmx = 0;      // max co-resident grids
   int grid64m = 0;                 // ... of the mean-constraint kernel
@@ -328,8 +335,7 @@ int ensure_events(cup2d_poisson* h) {
 int ensure_scratch(cup2d_poisson* h) {
   int st;
   const int g = std::max(h->grid64, h->gridmx);
-  if ((st = h->red.ensure((int64_t)kRedWords * std::max(g, 1))) || (st = h->bar.ensure(1)) ||
-      (st = h->abort_flag.ensure(1)) || (st = h->dstats.ensure(1)))
+  if ((st = h->red.ensure((int64_t)kRedWords * std::max(g, 1))) || (st = h->ctl.ensure(1)))
     return st;
   return CUP2D_OK;
 }
@@ -354,7 +360,7 @@ int ensure_mixed(cup2d_poisson* h) {
 }
 
 void fill_stats(const cup2d_poisson* h, int launch_status, float ms, cup2d_solve_stats* out) {
-  const DevStats& d = *h->hstats;
+  const DevStats& d = h->hctl->stats;
   out->status = launch_status != CUP2D_OK ? launch_status : d.status;
   out->iterations = d.iterations;
   out->restarts = d.restarts;
@@ -595,11 +601,9 @@ int handle_destroy_idle(cup2d_poisson* h) {
                           &h->f_nu, &h->f_t, &h->f_z, &h->f_z2};
   for (auto* b : f32) b->release();
   h->err.release();
-  h->bar.release();
-  h->abort_flag.release();
-  h->dstats.release();
+  h->ctl.release();
   h->prof.release();
-  if (h->hstats) cudaFreeHost(h->hstats);
+  if (h->hctl) cudaFreeHost(h->hctl);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->stream && h->owns_stream) cudaStreamDestroy(h->stream);
@@ -619,9 +623,7 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
   const cup2d_solve_opts& o = h->opts;
   int st;
   if ((st = ensure_scratch(h))) return st;
-  if (cudaMemsetAsync(h->bar.p, 0, sizeof(unsigned), s) != cudaSuccess ||
-      cudaMemsetAsync(h->abort_flag.p, 0, sizeof(int), s) != cudaSuccess)
-    return CUP2D_CUDA_ERROR;
+  if (cudaMemsetAsync(h->ctl.p, 0, offsetof(SolveCtl, stats), s) != cudaSuccess) return CUP2D_CUDA_ERROR;
   const unsigned long long tns = (unsigned long long)o.timeout_ms * 1000000ull;
   // the barrier counter counts arrivals of the whole solve in 32 bits
   // bMeanConstraint: row of cell (0,0) of the leaf at the domain's corner
@@ -646,8 +648,8 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
   }
   // the pinned statistics record is allocated when statistics are first
   // asked for (a page-locked allocation serialises the device's streams)
-  if (stats && !h->hstats && cudaMallocHost(&h->hstats, sizeof(DevStats)) != cudaSuccess) {
-    h->hstats = nullptr;
+  if (stats && !h->hctl && cudaMallocHost(&h->hctl, sizeof(SolveCtl)) != cudaSuccess) {
+    h->hctl = nullptr;
     return CUP2D_OOM;
   }
   if (stats && (st = ensure_events(h))) return st;
@@ -660,8 +662,8 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     a.prob.b = d_b;
     a.prob.x = d_x;
     a.prob.xo = h->xo.p;
-    a.prob.stats = h->dstats.p;
-    a.abort_flag = h->abort_flag.p;
+    a.prob.stats = &h->ctl.p->stats;
+    a.abort_flag = &h->ctl.p->abort_flag;
     a.sp = SolveParams{o.tol_abs, o.tol_rel, o.reliable_delta, o.max_restarts, o.max_iter, o.subtract_mean,
                        o.reliable_restart};
     a.timeout_ns = tns;
@@ -672,8 +674,8 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     a.prob.b = d_b;
     a.prob.x = d_x;
     a.prob.xo = h->xo.p;
-    a.prob.stats = h->dstats.p;
-    a.abort_flag = h->abort_flag.p;
+    a.prob.stats = &h->ctl.p->stats;
+    a.abort_flag = &h->ctl.p->abort_flag;
     a.sp = SolveParams{o.tol_abs, o.tol_rel, 0.0, o.max_restarts, o.max_iter, o.subtract_mean, 0};
     a.timeout_ns = tns;
     e = launch_bicgstab_cluster(a, cluster, s);
@@ -681,10 +683,10 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     if ((st = ensure_mixed(h))) return st;
     SolveArgsMixed a{};
     a.prob = ProblemMixed{h->mesh.view(), d_b, d_x, h->xo.p, h->f_r.p, h->f_rh.p, h->f_p.p, h->f_nu.p,
-                          h->f_t.p, h->f_z.p, h->f_z2.p, h->dstats.p};
+                          h->f_t.p, h->f_z.p, h->f_z2.p, &h->ctl.p->stats};
     a.red = h->red.p;
-    a.bar = h->bar.p;
-    a.abort_flag = h->abort_flag.p;
+    a.bar = &h->ctl.p->bar;
+    a.abort_flag = &h->ctl.p->abort_flag;
     a.sp = SolveParams{o.tol_abs, o.tol_rel, o.reliable_delta, o.max_restarts, o.max_iter, o.subtract_mean,
                        o.reliable_restart, mean_row};
     a.timeout_ns = tns;
@@ -694,10 +696,10 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
     if ((st = ensure_fp64(h))) return st;
     SolveArgs64 a{};
     a.prob = Problem64{h->mesh.view(), d_b, d_x, h->xo.p, h->r.p, h->rh.p, h->p.p, h->nu.p, h->t.p, h->z.p,
-                       h->z2.p, h->dstats.p};
+                       h->z2.p, &h->ctl.p->stats};
     a.red = h->red.p;
-    a.bar = h->bar.p;
-    a.abort_flag = h->abort_flag.p;
+    a.bar = &h->ctl.p->bar;
+    a.abort_flag = &h->ctl.p->abort_flag;
     a.sp = SolveParams{o.tol_abs, o.tol_rel, 0.0, o.max_restarts, o.max_iter, o.subtract_mean, 0, mean_row};
     a.timeout_ns = tns;
     a.prof = prof;
@@ -705,15 +707,13 @@ int cup2d_poisson_solve_device(cup2d_poisson* h, const double* d_b, double* d_x,
   }
   if (e != cudaSuccess) return from_cuda(e);
   if (!stats) return CUP2D_OK;
-  int habort = 0;
   cudaEventRecord(h->ev1, s);
-  if (cudaMemcpyAsync(h->hstats, h->dstats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaMemcpyAsync(&habort, h->abort_flag.p, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  if (cudaMemcpyAsync(h->hctl, h->ctl.p, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return CUP2D_CUDA_ERROR;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-  fill_stats(h, habort ? CUP2D_TIMEOUT : CUP2D_OK, ms, stats);
+  fill_stats(h, h->hctl->abort_flag ? CUP2D_TIMEOUT : CUP2D_OK, ms, stats);
   return stats->status == CUP2D_TIMEOUT ? CUP2D_TIMEOUT : CUP2D_OK;
 }
 
@@ -1578,14 +1578,7 @@ int handle_stage(cup2d_poisson* h, double** d_b, double** d_x) {
   return CUP2D_OK;
 }
 
-namespace {
-struct RawStats {
-  DevStats d;
-  int aborted;
-};
-}  // namespace
-
-size_t handle_stats_bytes() { return sizeof(RawStats); }
+size_t handle_stats_bytes() { return sizeof(SolveCtl); }
 
 int handle_solve_async(cup2d_poisson* h, const double* d_b, double* d_x, cudaStream_t stream, void* raw) {
   if (!raw) return CUP2D_INVALID_ARGUMENT;
@@ -1595,17 +1588,15 @@ int handle_solve_async(cup2d_poisson* h, const double* d_b, double* d_x, cudaStr
   }
   const int st = cup2d_poisson_solve_device(h, d_b, d_x, nullptr, stream);
   if (st) return st;
-  auto* rs = static_cast<RawStats*>(raw);
-  if (cudaMemcpyAsync(&rs->d, h->dstats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-      cudaMemcpyAsync(&rs->aborted, h->abort_flag.p, sizeof(int), cudaMemcpyDeviceToHost, stream) != cudaSuccess)
-    return CUP2D_CUDA_ERROR;
-  return CUP2D_OK;
+  return cudaMemcpyAsync(raw, h->ctl.p, sizeof(SolveCtl), cudaMemcpyDeviceToHost, stream) == cudaSuccess
+             ? CUP2D_OK
+             : CUP2D_CUDA_ERROR;
 }
 
 void handle_stats_from_raw(const void* raw, double solve_ms, cup2d_solve_stats* out) {
-  const auto* rs = static_cast<const RawStats*>(raw);
-  const DevStats& d = rs->d;
-  out->status = rs->aborted ? CUP2D_TIMEOUT : d.status;
+  const auto* rs = static_cast<const SolveCtl*>(raw);
+  const DevStats& d = rs->stats;
+  out->status = rs->abort_flag ? CUP2D_TIMEOUT : d.status;
   out->iterations = d.iterations;
   out->restarts = d.restarts;
   out->refinements = d.refinements;
