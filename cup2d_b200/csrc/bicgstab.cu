@@ -3,9 +3,10 @@
 //
 //   k_bicgstab64     plain FP64: the drop-in form of BiCGSTABSolver::main
 //                    (source/Poisson/BiCGSTAB.cu:412-620)
-//   k_bicgstab_mixed FP32 Krylov vectors and split-TF32 tensor-core P^-1;
-//                    FP64 solution update, FP64 true-residual replacement
-//                    ("reliable updates") and FP64 convergence test
+//   k_bicgstab_mixed FP32 Krylov vectors and FP32 P^-1; FP64 solution
+//                    update, FP64 true-residual replacement ("reliable
+//                    updates") and FP64 convergence test
+// P^-1 is applied as sine transforms in registers (sine_solve.cuh).
 //
 // The reference runs each iteration as ~25 library launches (cuSPARSE COO
 // SpMV, cuBLAS dot/nrm2/axpy/scal/Idamax/Dgemm), 8 one-thread scalar kernels
@@ -231,6 +232,42 @@ __device__ __forceinline__ bool computes_row(const MeshView& M, int row, int b0,
   return owns_row(row, b0, b1);
 }
 
+// The vectors only their own CTA touches between true residuals, p and x, stay
+// in shared memory for as many of its chunks as fit: the passes of a large solve
+// run at the rate of L2 (8-11 TB/s), and p is 2 of pass A's 5 streams, x 2 of pass
+// E's 8.  On 20,834 blocks this measured FP64 48.5 -> 41.8 us, mixed 38.1 -> 36.5 us
+// an iteration.  A chunk of p is a slot of kSlotBytes (16 bytes a lane, the fragment
+// layout), a chunk of x CB slots in cell order.  p fills the slots first.
+constexpr int kSlotBytes = 512;
+
+template <class T, bool RES>
+struct Resident {
+  T* p;       // chunk c < np of p
+  double* x;  // chunk c < nx of x
+  int np, nx;
+  bool any;   // whether the launch has slots at all (the same for the team)
+  __device__ __forceinline__ Resident(unsigned char* base, int slots, int b0, int b1) {
+    const int nch = (b1 - b0 + Frag<T>::CB - 1) / Frag<T>::CB;
+    np = RES ? min(nch, slots) : 0;
+    nx = RES ? min(nch, (slots - np) / Frag<T>::CB) : 0;
+    p = reinterpret_cast<T*>(base);
+    x = reinterpret_cast<double*>(base + (size_t)np * kSlotBytes);
+    any = RES && slots > 0;
+  }
+  __device__ __forceinline__ T* p_at(int c, int lane) const { return p + (c * 32 + lane) * Frag<T>::N; }
+  // the two functions below copy whole chunks; all threads, then synchronise
+  __device__ __forceinline__ void fetch_x(const double* __restrict__ g, int b0, int b1) const {
+    const int n = min(nx * Frag<T>::CB, b1 - b0) * kBLEN;
+    for (int i = 2 * (int)threadIdx.x; i < n; i += 2 * kSolveThreads)
+      *reinterpret_cast<double2*>(x + i) = __ldcg(reinterpret_cast<const double2*>(g + b0 * kBLEN + i));
+  }
+  __device__ __forceinline__ void put_x(double* __restrict__ g, int b0, int b1) const {
+    const int n = min(nx * Frag<T>::CB, b1 - b0) * kBLEN;
+    for (int i = 2 * (int)threadIdx.x; i < n; i += 2 * kSolveThreads)
+      *reinterpret_cast<double2*>(g + b0 * kBLEN + i) = *reinterpret_cast<const double2*>(x + i);
+  }
+};
+
 struct IterState {
   double rho, nr, nrh;  // (rhat,r), |r|^2, |rhat|^2 of the current residual
   double err_init;      // L-inf norm the relative test divides by
@@ -385,9 +422,9 @@ struct MixedCtx {  // what the reliable update needs
 // X the solution type; RU enables the mixed form's true-residual
 // replacement; MC the mean constraint (FP64 only); AHEAD the operands of
 // passes A and C one chunk ahead.  Returns false if a barrier gave up.
-template <class T, bool RU, bool MC, bool AHEAD>
+template <class T, bool RU, bool MC, bool AHEAD, bool RES>
 __device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, const Problem<T>& V,
-                              int b0, int b1, int r0, int r1, const SolveParams& sp,
+                              const Resident<T, RES>& R, int b0, int b1, int r0, int r1, const SolveParams& sp,
                               const MixedCtx& mx, IterState& st) {
   static_assert(!(MC && RU), "the mean constraint runs in the FP64 form only");
   using X = double;
@@ -430,25 +467,27 @@ __device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, con
     // that the loads overlap it.
     {
       T rr[FN], pp[FN], nn[FN];
-      auto load = [&](int blk) {
-        const int nv = b1 - blk;
+      auto load = [&](int c) {
+        const int blk = b0 + c * CB, nv = b1 - blk;
         ld_frag<T>(V.r, blk, nv, lane, rr);
         if (!zero_pnu) {
-          ld_frag<T>(V.p, blk, nv, lane, pp);
+          if (RES && c < R.np) lds16<FN>(R.p_at(c, lane), pp);
+          else ld_frag<T>(V.p, blk, nv, lane, pp);
           ld_frag<T>(V.nu, blk, nv, lane, nn);
         }
       };
-      int blk = b0 + w * CB;
-      if (AHEAD && blk < b1) load(blk);
-      for (; blk < b1; blk += kWarps * CB) {
-        if (!AHEAD) load(blk);
-        const int nv = b1 - blk;
+      const int nch = (b1 - b0 + CB - 1) / CB;
+      if (AHEAD && w < nch) load(w);
+      for (int c = w; c < nch; c += kWarps) {
+        if (!AHEAD) load(c);
+        const int blk = b0 + c * CB, nv = b1 - blk;
         T pv[FN];
 #pragma unroll
         for (int k = 0; k < FN; ++k) pv[k] = zero_pnu ? rr[k] : rr[k] + tb_beta * (pp[k] - tb_omega * nn[k]);
         if (restart_now) st_frag<T>(V.rh, blk, nv, lane, rr);
-        st_frag<T>(V.p, blk, nv, lane, pv);
-        if (AHEAD && blk + kWarps * CB < b1) load(blk + kWarps * CB);
+        if (RES && c < R.np) stv<FN>(R.p_at(c, lane), pv);
+        else st_frag<T>(V.p, blk, nv, lane, pv);
+        if (AHEAD && c + kWarps < nch) load(c + kWarps);
         pin.apply(pv, scratch, lane);
         st_frag<T>(V.z, blk, nv, lane, pv);
       }
@@ -548,7 +587,17 @@ __device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, con
         const int i0 = blk * kBLEN + L.cell0;
         X xv[LV];
         T zv[LV], z2v[LV], sv[LV], tv[LV], rhv[LV];
-        ldv<LV>(V.x + i0, xv);
+        double* const xs = R.x + (c * CB + L.bl) * kBLEN + L.cell0;  // where chunk c of x is resident
+        if (RES && c < R.nx) {
+#pragma unroll
+          for (int k = 0; k < LV; k += 2) {
+            const double2 a = *reinterpret_cast<const double2*>(xs + k);
+            xv[k] = a.x;
+            xv[k + 1] = a.y;
+          }
+        } else {
+          ldv<LV>(V.x + i0, xv);
+        }
         ldv<LV>(V.z + i0, zv);
         ldv<LV>(V.z2 + i0, z2v);
         ldv<LV>(V.r + i0, sv);
@@ -567,7 +616,7 @@ __device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, con
           v[2] += dprod(rn[k], rn[k]);
           v[3] += dprod(rhv[k], rhv[k]);
         }
-        stv<LV>(V.x + i0, xn);
+        stv<LV>(RES && c < R.nx ? xs : V.x + i0, xn);
         stv<LV>(V.r + i0, rn);
       }
       if (!B.reduce<4>(v, 0x1u, 5)) return false;
@@ -590,7 +639,12 @@ __device__ bool bicgstab_loop(Smem<T>& sm, Team& B, const SineSolve<T>& pin, con
       // or a sweep stalls for kMaxSweep iterations
       if (claims || sqrt(nr) < mx.delta * rmax_since || since >= kMaxSweep) {
         since = 0;
-        // pass E's barrier already ordered every CTA's x update before this
+        // pass E's barrier already ordered every CTA's x update before this,
+        // but for what is resident
+        if (RES && R.any) {
+          R.put_x(V.x, b0, b1);
+          if (!B.sync(6)) return false;
+        }
         if (!true_residual(sm, B, M, mx.b, mx.mean_b, V.x, V.r, V.rh, mx.restart, b0, b1, r0, r1, 6)) return false;
         ++st.updates;
         refreshed = true;
@@ -678,6 +732,14 @@ __device__ __forceinline__ void take_best(bool best_is_x, double* __restrict__ x
   }
 }
 
+// The kernels' dynamic shared memory: Smem<T>, then the resident slots.
+extern __shared__ __align__(16) unsigned char g_solve_smem[];
+static_assert(sizeof(Smem<float>) % 16 == 0 && sizeof(Smem<double>) % 16 == 0, "16-byte slots");
+template <class T>
+__device__ __forceinline__ Smem<T>& solve_smem() {
+  return *reinterpret_cast<Smem<T>*>(g_solve_smem);
+}
+
 // ============================================ one problem, one team ========
 
 __device__ __forceinline__ void write_stats(const Team& B, DevStats* stats, const IterState& st, int refinements,
@@ -697,11 +759,12 @@ __device__ __forceinline__ void write_stats(const Team& B, DevStats* stats, cons
 // (BiCGSTAB.cu:412-620) and the mean removal (ExpAMRSolver.cpp:383-415).
 // [b0,b1) is this CTA's block range, [r0,r1) its explicit rows.
 // MC: the mean constraint (sp.mean_row).
-template <bool MC, bool AHEAD = true>
+template <bool MC, bool RES, bool AHEAD = true>
 __device__ bool solve_fp64(Smem<double>& sm, Team& B, const SineSolve<double>& pin, const Problem64& pr,
-                           const SolveParams& sp, int b0, int b1, int r0,
-                           int r1) {
+                           const SolveParams& sp, int slots, int b0, int b1, int r0, int r1) {
   const MeshView& M = pr.M;
+  const Resident<double, RES> R(g_solve_smem + sizeof(Smem<double>), slots, b0, b1);
+  if constexpr (RES) R.fetch_x(pr.x, b0, b1);  // read after the first reduction's barriers
   double x0sum = 0.0;  // MC: sum h^2 x0, the mean row of A x0
   if constexpr (MC) {
     const double v[1] = {hsum_part(M, pr.x, b0, b1)};
@@ -769,8 +832,12 @@ __device__ bool solve_fp64(Smem<double>& sm, Team& B, const SineSolve<double>& p
   st.best_is_x = true;
   st.status = CUP2D_NOT_CONVERGED;
   const MixedCtx none{};
-  if (!bicgstab_loop<double, false, MC, AHEAD>(sm, B, pin, pr, b0, b1, r0, r1, sp, none, st))
+  if (!bicgstab_loop<double, false, MC, AHEAD, RES>(sm, B, pin, pr, R, b0, b1, r0, r1, sp, none, st))
     return false;
+  if (RES && R.any && st.best_is_x) {
+    R.put_x(pr.x, b0, b1);
+    __syncthreads();
+  }
   take_best(st.best_is_x, pr.x, pr.xo, b0, b1);
   if (sp.subtract_mean && !subtract_mean(sm, B, M, pr.x, b0, b1)) return false;
   write_stats(B, pr.stats, st, 0, st.err_opt, norm_ax0);
@@ -778,9 +845,11 @@ __device__ bool solve_fp64(Smem<double>& sm, Team& B, const SineSolve<double>& p
 }
 
 // Mixed-precision solve of one problem by the team.
+template <bool RES>
 __device__ bool solve_mixed(Smem<float>& sm, Team& B, const SineSolve<float>& pin, const ProblemMixed& pr,
-                            const SolveParams& sp, int b0, int b1, int r0,
-                            int r1) {
+                            const SolveParams& sp, int slots, int b0, int b1, int r0, int r1) {
+  const Resident<float, RES> R(g_solve_smem + sizeof(Smem<float>), slots, b0, b1);
+  if constexpr (RES) R.fetch_x(pr.x, b0, b1);  // read after the first reduction's barriers
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // Neumann compatibility: project b to zero sum (sum b / n)
   {
@@ -814,7 +883,7 @@ __device__ bool solve_mixed(Smem<float>& sm, Team& B, const SineSolve<float>& pi
   const bool done0 = st.err_true <= sp.tol_abs || st.err_true == 0.0;
   if (done0) {
     st.status = CUP2D_OK;
-  } else if (!bicgstab_loop<float, true, false, true>(sm, B, pin, pr, b0, b1, r0, r1, sp, mx, st)) {
+  } else if (!bicgstab_loop<float, true, false, true, RES>(sm, B, pin, pr, R, b0, b1, r0, r1, sp, mx, st)) {
     return false;
   }
   take_best(st.best_is_x, pr.x, pr.xo, b0, b1);
@@ -824,15 +893,6 @@ __device__ bool solve_mixed(Smem<float>& sm, Team& B, const SineSolve<float>& pi
 }
 
 }  // namespace
-
-// The kernels' shared memory (P^-1, staging tiles and SpMV rings, reduction
-// scratch) is above the 48 KB of a static allocation: dynamic, sized
-// sizeof(Smem<T>) at every launch.
-extern __shared__ __align__(16) unsigned char g_solve_smem[];
-template <class T>
-__device__ __forceinline__ Smem<T>& solve_smem() {
-  return *reinterpret_cast<Smem<T>*>(g_solve_smem);
-}
 
 // ====================================================== single solves =====
 
@@ -850,7 +910,7 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab64(c
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<false>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
+  solve_fp64<false, true>(sm, B, pin, S.prob, S.sp, S.nslots, b0, b1, r0, r1);
 }
 
 // With bMeanConstraint: the same solve on the system whose row S.sp.mean_row
@@ -865,7 +925,7 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm)
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<true>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
+  solve_fp64<true, true>(sm, B, pin, S.prob, S.sp, S.nslots, b0, b1, r0, r1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab_mixed(const __grid_constant__ SolveArgsMixed S) {
@@ -877,7 +937,7 @@ __global__ void __launch_bounds__(kSolveThreads, kSolveCtasPerSm) k_bicgstab_mix
   SineSolve<float> pin;
   pin.init();
   __syncthreads();
-  solve_mixed(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
+  solve_mixed<true>(sm, B, pin, S.prob, S.sp, S.nslots, b0, b1, r0, r1);
 }
 
 
@@ -893,7 +953,7 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
   SineSolve<double> pin;
   pin.init();
   __syncthreads();
-  solve_fp64<false>(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
+  solve_fp64<false, false>(sm, B, pin, S.prob, S.sp, 0, b0, b1, r0, r1);
 }
 
 __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
@@ -906,7 +966,7 @@ __global__ void __launch_bounds__(kSolveThreads, kServedCtasPerSm)
   SineSolve<float> pin;
   pin.init();
   __syncthreads();
-  solve_mixed(sm, B, pin, S.prob, S.sp, b0, b1, r0, r1);
+  solve_mixed<false>(sm, B, pin, S.prob, S.sp, 0, b0, b1, r0, r1);
 }
 
 // ========================================================= batches ========
@@ -948,14 +1008,14 @@ __device__ __forceinline__ void batch_body(const BatchArgs& A) {
       const ProblemMixed& pr = A.pmx[p];
       const int b0 = share(pr.M.nb, rank, team), b1 = share(pr.M.nb, rank + 1, team);
       const int r0 = share(pr.M.R, rank, team), r1 = share(pr.M.R, rank + 1, team);
-      ok = solve_mixed(sm, B, pin, pr, A.sp, b0, b1, r0, r1);
+      ok = solve_mixed<false>(sm, B, pin, pr, A.sp, 0, b0, b1, r0, r1);
     } else {
       const Problem64& pr = A.p64[p];
       const int b0 = share(pr.M.nb, rank, team), b1 = share(pr.M.nb, rank + 1, team);
       const int r0 = share(pr.M.R, rank, team), r1 = share(pr.M.R, rank + 1, team);
       // at 80 registers the operands held ahead are spilled: 23.3 -> 22.3 ms
       // for 40 iterations of 200 problems on teams of 8 without them
-      ok = solve_fp64<false, false>(sm, B, pin, pr, A.sp, b0, b1, r0, r1);
+      ok = solve_fp64<false, false, false>(sm, B, pin, pr, A.sp, 0, b0, b1, r0, r1);
     }
     if (!ok) return;
     if (rank == 0 && threadIdx.x == 0) {
@@ -986,65 +1046,93 @@ const void* const kSolveFns[kNumSolveFns] = {(const void*)k_bicgstab64,        (
 const int kSolveFnCtas[kNumSolveFns] = {kSolveCtasPerSm,  kSolveCtasPerSm,  kBatch64CtasPerSm, kBatchMixedCtasPerSm,
                                         kSolveCtasPerSm,  kServedCtasPerSm, kServedCtasPerSm};
 
-size_t smem_bytes(const void* fn) {
+int fn_index(const void* fn) {
+  int k = 0;
+  while (k < kNumSolveFns && kSolveFns[k] != fn) ++k;
+  return k;
+}
+
+// The kernels with resident slots.
+bool resident(const void* fn) {
+  return fn == (const void*)k_bicgstab64 || fn == (const void*)k_bicgstab64_mean || fn == (const void*)k_bicgstab_mixed;
+}
+
+// Shared memory of a solve kernel beside its resident slots.
+size_t base_smem(const void* fn) {
   return (fn == kSolveFns[1] || fn == kSolveFns[3] || fn == kSolveFns[6]) ? sizeof(Smem<float>)
                                                                            : sizeof(Smem<double>);
 }
 
-// Allows the dynamic shared memory of a solve kernel on the current device
-// (once per device and kernel) and asks for the smallest shared-memory
-// carve-out that holds the CTAs per SM it is built for (kSolveFnCtas), so
-// that the rest of the
-// unified array stays L1.
-cudaError_t allow_smem(const void* fn) {
-  static unsigned done[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  int k = 0;
-  while (k < kNumSolveFns && kSolveFns[k] != fn) ++k;
-  const unsigned bit = 1u << k;
-  if (dev >= 0 && dev < 64 && (__atomic_load_n(&done[dev], __ATOMIC_ACQUIRE) & bit)) return cudaSuccess;
-  const size_t bytes = smem_bytes(fn);
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  int per_sm = 0, reserved = 0;
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-  if (e == cudaSuccess && per_sm > 0) {
-    const int ctas = k < kNumSolveFns ? kSolveFnCtas[k] : kSolveCtasPerSm;
-    const size_t need = (size_t)ctas * (bytes + (size_t)reserved);
-    const int pct = (int)std::min<size_t>(100, (need * 100 + per_sm - 1) / (size_t)per_sm);
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+// What a solve kernel may use on a device, queried once per device and kernel
+// (handles are created often, e.g. by a server): the largest co-resident grid
+// and the resident slots of a CTA.  The plain single solves fill their share of
+// the SM's shared memory with slots.  The batches and the served forms have none:
+// their vectors stream from HBM and the tables live off L1, which the slots
+// would take (512 problems, mixed: 597 ms without, 634 ms with them).
+struct FnLimits {
+  int grid = 0, slots = 0;
+};
+
+cudaError_t query_limits(const void* fn, int dev, FnLimits& out) {
+  int per_sm = 0, reserved = 0, optin = 0, sms = 0, ctas = 0;
+  cudaError_t e;
+  if ((e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    return e;
+  const int want = kSolveFnCtas[fn_index(fn)];
+  const size_t base = base_smem(fn);
+  const size_t most = std::min<size_t>(optin, (size_t)per_sm / want - (size_t)reserved);
+  const int slots = resident(fn) && most > base ? (int)((most - base) / kSlotBytes) : 0;
+  const size_t bytes = base + (size_t)slots * kSlotBytes;
+  const int pct = (int)std::min<size_t>(100, (want * (bytes + (size_t)reserved) * 100 + per_sm - 1) / (size_t)per_sm);
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct)) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, kSolveThreads, bytes)) != cudaSuccess)
+    return e;
+  out.grid = sms * ctas;
+  out.slots = slots;
+  return cudaSuccess;
+}
+
+FnLimits fn_limits(const void* fn, int device) {
+  static std::atomic<uint64_t> cache[64][kNumSolveFns];
+  const int k = fn_index(fn);
+  const bool keep = device >= 0 && device < 64;
+  if (keep) {
+    const uint64_t v = cache[device][k].load(std::memory_order_acquire);
+    if (v) return FnLimits{(int)(v >> 32), (int)(uint32_t)v};
   }
-  if (e == cudaSuccess && dev >= 0 && dev < 64) __atomic_fetch_or(&done[dev], bit, __ATOMIC_ACQ_REL);
-  return e;
-}
-
-// The largest co-resident grid of a solve kernel on a device: queried once
-// per device and kernel (handles are created often, e.g. by a server).
-int coop_grid_query(const void* fn, int device) {
-  int sms = 0, per_sm = 0, cur = 0;
-  if (cudaGetDevice(&cur) != cudaSuccess) return 0;
-  if (cur != device && cudaSetDevice(device) != cudaSuccess) return 0;
-  const bool ok = allow_smem(fn) == cudaSuccess &&
-                  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
-                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSolveThreads, smem_bytes(fn)) ==
-                      cudaSuccess;
+  FnLimits l;
+  int cur = 0;
+  if (cudaGetDevice(&cur) != cudaSuccess) return FnLimits{};
+  if (cur != device && cudaSetDevice(device) != cudaSuccess) return FnLimits{};
+  const bool ok = query_limits(fn, device, l) == cudaSuccess;
   if (cur != device) cudaSetDevice(cur);
-  return ok ? sms * per_sm : 0;
+  if (!ok) return FnLimits{};
+  if (keep && l.grid > 0)
+    cache[device][k].store(((uint64_t)l.grid << 32) | (uint32_t)l.slots, std::memory_order_release);
+  return l;
 }
 
-int coop_grid(const void* fn, int device) {
-  static std::atomic<int> cache[64][kNumSolveFns];
-  int k = 0;
-  while (k < kNumSolveFns && kSolveFns[k] != fn) ++k;
-  if (device < 0 || device >= 64 || k == kNumSolveFns) return coop_grid_query(fn, device);
-  int g = cache[device][k].load(std::memory_order_acquire);
-  if (g > 0) return g;
-  g = coop_grid_query(fn, device);
-  if (g > 0) cache[device][k].store(g, std::memory_order_release);
-  return g;
+// The kernel's limits on the current device; its attributes are set.
+cudaError_t current_limits(const void* fn, FnLimits& l) {
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  l = fn_limits(fn, dev);
+  return l.grid > 0 ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
+
+// Slots a solve of nb blocks by `grid` CTAs can use: p and x of the largest
+// share.
+template <class T>
+int used_slots(int64_t nb, int grid, int slots) {
+  const int64_t nch = ((nb + grid - 1) / grid + Frag<T>::CB - 1) / Frag<T>::CB;
+  return (int)std::min<int64_t>(slots, nch * (1 + Frag<T>::CB));
+}
+
+int coop_grid(const void* fn, int device) { return fn_limits(fn, device).grid; }
 }  // namespace
 
 int max_coop_grid_fp64(int device, bool served) {
@@ -1056,21 +1144,27 @@ int max_coop_grid_mixed(int device, bool served) {
 
 int max_coop_grid_mean(int device) { return coop_grid((const void*)k_bicgstab64_mean, device); }
 
-cudaError_t launch_bicgstab64(const SolveArgs64& a, int grid, cudaStream_t s, bool served) {
-  void* args[] = {const_cast<SolveArgs64*>(&a)};
+cudaError_t launch_bicgstab64(SolveArgs64& a, int grid, cudaStream_t s, bool served) {
+  void* args[] = {&a};
   const void* fn = a.sp.mean_row >= 0 ? (const void*)k_bicgstab64_mean
                    : served           ? (const void*)k_bicgstab64_served
                                       : (const void*)k_bicgstab64;
-  if (cudaError_t e = allow_smem(fn)) return e;
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolveThreads), args, sizeof(Smem<double>), s);
+  FnLimits l;
+  if (cudaError_t e = current_limits(fn, l)) return e;
+  a.nslots = used_slots<double>(a.prob.M.nb, grid, l.slots);
+  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolveThreads), args,
+                                     sizeof(Smem<double>) + (size_t)a.nslots * kSlotBytes, s);
 }
 
-cudaError_t launch_bicgstab_mixed(const SolveArgsMixed& a, int grid, cudaStream_t s, bool served) {
-  void* args[] = {const_cast<SolveArgsMixed*>(&a)};
+cudaError_t launch_bicgstab_mixed(SolveArgsMixed& a, int grid, cudaStream_t s, bool served) {
+  void* args[] = {&a};
   if (a.sp.mean_row >= 0) return cudaErrorInvalidValue;  // FP64 only
   const void* fn = served ? (const void*)k_bicgstab_mixed_served : (const void*)k_bicgstab_mixed;
-  if (cudaError_t e = allow_smem(fn)) return e;
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolveThreads), args, sizeof(Smem<float>), s);
+  FnLimits l;
+  if (cudaError_t e = current_limits(fn, l)) return e;
+  a.nslots = used_slots<float>(a.prob.M.nb, grid, l.slots);
+  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolveThreads), args,
+                                     sizeof(Smem<float>) + (size_t)a.nslots * kSlotBytes, s);
 }
 
 int max_coop_grid_batch(int device, bool mixed) {
@@ -1082,14 +1176,15 @@ int max_coop_grid_batch(int device, bool mixed) {
 cudaError_t launch_bicgstab_batch(const BatchArgs& a, int grid, bool mixed, cudaStream_t s) {
   void* args[] = {const_cast<BatchArgs*>(&a)};
   const void* fn = mixed ? (const void*)k_bicgstab_batch_mixed : (const void*)k_bicgstab_batch64;
-  if (cudaError_t e = allow_smem(fn)) return e;
+  FnLimits l;
+  if (cudaError_t e = current_limits(fn, l)) return e;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kSolveThreads);
-  cfg.dynamicSmemBytes = smem_bytes(fn);
+  cfg.dynamicSmemBytes = base_smem(fn);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

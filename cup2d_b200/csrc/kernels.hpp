@@ -130,6 +130,7 @@ struct SolveArgs64 {
   SolveParams sp;
   unsigned long long timeout_ns;
   unsigned long long* prof;  // per-CTA phase timers, or null
+  int nslots;                // resident slots in shared memory (set by the launch)
 };
 
 // Mixed precision: FP32 Krylov vectors, FP64 solution and true residual.
@@ -141,6 +142,7 @@ struct SolveArgsMixed {
   SolveParams sp;
   unsigned long long timeout_ns;
   unsigned long long* prof;  // per-CTA phase timers, or null
+  int nslots;                // resident slots in shared memory (set by the launch)
 };
 
 // Many problems in one launch: groups of `team` CTAs take problems from a
@@ -209,8 +211,8 @@ int max_coop_grid_fp64(int device, bool served = false);
 int max_coop_grid_mixed(int device, bool served = false);
 // With a.sp.mean_row >= 0 the FP64 launch runs the mean-constraint variant;
 // the mixed form has none.
-cudaError_t launch_bicgstab64(const SolveArgs64& a, int grid, cudaStream_t s, bool served = false);
-cudaError_t launch_bicgstab_mixed(const SolveArgsMixed& a, int grid, cudaStream_t s, bool served = false);
+cudaError_t launch_bicgstab64(SolveArgs64& a, int grid, cudaStream_t s, bool served = false);
+cudaError_t launch_bicgstab_mixed(SolveArgsMixed& a, int grid, cudaStream_t s, bool served = false);
 int max_coop_grid_mean(int device);
 int max_coop_grid_batch(int device, bool mixed);
 cudaError_t launch_bicgstab_batch(const BatchArgs& a, int grid, bool mixed, cudaStream_t s);
@@ -296,7 +298,7 @@ cudaError_t launch_rhs_fourier(const ForestView& F, int kmax, const double* coef
 int64_t wmean_partials(int64_t nb);
 cudaError_t launch_add_pold(double* pres, const double* pold, const double* hblk, int64_t nb, double* partial,
                             cudaStream_t s);
-// Pressure projection around the solve (projection.cu), one thread per cell.
+// Pressure projection around the solve (projection.cu), one warp per block.
 // Velocity-like fields hold (u, v) per cell, interleaved, in block-major
 // cell order; scalars one double per cell.
 //   rhs:  tmp = h/(2dt) (central div vel - chi central div udef)  (vel set)

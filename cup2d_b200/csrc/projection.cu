@@ -9,8 +9,8 @@
 //   updatePressureRHS1 (:399-456)  TMP -= ((p_W + p_E) + (p_S + p_N)) - 4 p
 //   pressureCorrection (:123-210)  tmpV = pFac (P_E - P_W, P_N - P_S),
 //                                  pFac = -0.5 dt h; V += tmpV (1/h)/h
-// Here one thread owns one cell and evaluates its formula in the same order,
-// reading its ghosts straight from the neighbouring blocks:
+// Here one warp owns a block, a lane two cells, and evaluates each cell's formula
+// in the same order, reading its ghosts straight from the neighbouring blocks:
 //   * same-level neighbour: the touching cell;
 //   * non-periodic domain edge: velocities flip the sign of the normal
 //     component (BlockLabDirichlet, source/Definitions.h:71-196, wall and
@@ -21,7 +21,7 @@
 //     with D1/D2 of ExpAMRSolver.h:268-300), evaluated on values:
 //     2/3 close - 1/5 far + 8/15 ((c + sT D1) + D2);
 //   * finer neighbours: the mean of the four fine cells the ghost covers.
-// The flux correction is folded into the coarse cell's own thread: after its
+// The flux correction is folded into the coarse cell's own lane: after its
 // formula it adds its own face value (the kernel's storedFace expression with
 // that ghost) plus the two fine cells' face values (the same expression from
 // the fine side, with their interpolated ghosts).  Cubism, which owns the labs
