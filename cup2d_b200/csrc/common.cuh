@@ -236,8 +236,9 @@ struct Team {
   __device__ __noinline__ bool exchange(int nv, unsigned is_max, int phase) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned n = size;
-    __syncthreads();
+    // read ahead of the barrier: behind it thread 0's wait advances epoch
     double* const set = slots + (size_t)(epoch & 1u) * kRedMax * n;
+    __syncthreads();
     if (w == 0) {
       if (lane < nv) {
         double acc = wred[0][lane];
