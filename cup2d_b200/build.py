@@ -21,7 +21,7 @@ SOURCES = ["assemble.cu", "adapt.cu", "bicgstab.cu", "bicgstab_cluster.cu", "cap
            "server.cu", "timestep.cu", "spmv_apply.cu", "problems.cpp", "forest.cpp"]
 # files whose arithmetic must round like a plain IEEE evaluation (no FMA)
 FILE_FLAGS = {"projection.cu": ["--fmad=false"]}
-HEADERS = ["common.cuh", "kernels.hpp", "spmv.cuh", "sine_solve.cuh", "handle_view.hpp", "forest.hpp"]
+HEADERS = ["common.cuh", "kernels.hpp", "spmv.cuh", "sine_solve.cuh", "cluster_team.cuh", "handle_view.hpp", "forest.hpp"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",

@@ -28,14 +28,16 @@
 // Copies of the neighbours' blocks pushed ahead of each SpMV, so that no load
 // left the CTA, measured no faster (their stores cost what the loads had).
 //
-// The CTAs of a cluster are co-resident and pass the same barriers; the
-// deadline is one of pass E's reduced quantities, so all CTAs leave together.
-// The polls of a reduction are bounded besides.
+// The CTAs of a cluster are co-resident and pass the same barriers.  All CTAs
+// leave together: at the deadline, which is one of pass E's reduced quantities,
+// or behind the next barrier when a reduction's bounded wait ran out in any of
+// them (cluster_team.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <atomic>
 
+#include "cluster_team.cuh"
 #include "common.cuh"
 #include "kernels.hpp"
 #include "sine_solve.cuh"
@@ -45,17 +47,8 @@ namespace cup2d {
 
 namespace {
 
-constexpr int kClThreads = 512;
-constexpr int kClWarps = kClThreads / 32;
-constexpr int kMaxCluster = 16;
 constexpr int kMaxSweep = 64;  // mixed: longest FP32 sweep between true residuals
-constexpr unsigned kMaxPolls = 1u << 23;  // bound of a reduction's wait, some 0.3 s
 
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, unsigned rank) {
-  uint32_t a;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-  return a;
-}
 // Loads through the cluster's shared memory.  The conditional ones are
 // predicated, not branched around: a chunk's and a row's loads then stay in
 // flight together (with branches an SpMV pass of one chunk a warp took 4.3k
@@ -96,34 +89,15 @@ __device__ __forceinline__ void ld_cluster2_if(bool p, uint32_t a, float (&v)[2]
                : "r"(a), "r"((unsigned)p));
 }
 constexpr uint32_t kCodes = 1u;  // neighbour entries up to here: 0 wall, 1 coarse/fine face
-// Two 64-bit words; each is written and read whole.
-__device__ __forceinline__ void st_cluster_words(uint32_t a, unsigned long long x, unsigned long long y) {
-  asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
-}
-__device__ __forceinline__ ulonglong2 ld_words(uint32_t a) {
-  ulonglong2 v;
-  asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cluster_sync() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 __device__ __forceinline__ double prod(double a, double b) { return a * b; }
 __device__ __forceinline__ double prod(float a, float b) { return (double)a * (double)b; }
 
 // Fixed part of a CTA's shared memory.
 struct ClHead {
-  double wred[kClWarps][kRedMax];
-  double out[2][kRedMax];                // the last two reductions' results
-  // the CTAs' partials, posted by each into every CTA: {tag, low half} and
-  // {tag, high half} of a double
-  alignas(16) ulonglong2 post[2][kRedMax][kMaxCluster];
-  double sine[32][4];                    // mixed: the FP64 block solve's constants per lane
-  unsigned nlong;                        // explicit rows longer than kRowWidth
-  int lost;                              // a partial did not arrive
+  ClusterPosts posts;
+  double sine[32][4];  // mixed: the FP64 block solve's constants per lane
+  unsigned nlong;      // explicit rows longer than kRowWidth
 };
 
 constexpr int kSlotBytes = 512;  // one chunk of one vector: 16 bytes a lane
@@ -209,7 +183,7 @@ template <class T>
 struct Cluster {
   static constexpr int CB = Frag<T>::CB, N = Frag<T>::N;
   const MeshView& M;
-  ClHead& head;
+  ClusterTeam team;
   Slots<T> K;
   T* z;           // [nbl * 64], block order
   double* y;      // [nbl * 64]
@@ -217,7 +191,6 @@ struct Cluster {
   const unsigned long long* mask;    // explicit rows of a block
   const uint32_t* addr;              // z of every block of the forest
   T* scratch;     // the warp's 512 bytes
-  unsigned rank, size;
   int r0, r1;     // explicit rows of the CTA's blocks, the first `kept` in shared memory:
   int kept;       // entry j of row i at [j * cap + i]
   int cap;
@@ -226,54 +199,6 @@ struct Cluster {
   const uint32_t* raddr;
   const T* lval;  // the long rows' further entries
   const uint32_t* laddr;
-  unsigned posts;
-
-  // Sums (bit q of is_max: maxima) of v over the cluster's threads, in out.
-  // Each CTA writes its partial, tagged, into every CTA's shared memory and
-  // waits for the others' in its own: one way across (a cluster barrier behind
-  // the same stores took 740 clocks on 8 CTAs and 1020 on 16).  A CTA posts
-  // after all its warps have finished the pass, so what follows may overwrite
-  // what the pass read; it orders no other data (that takes cluster_sync).
-  // The wait is bounded: past it head.lost is set, and the caller leaves.
-  template <int NV>
-  __device__ __forceinline__ bool reduce(const double (&v)[NV], unsigned is_max, double (&out)[NV]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    warp_partials<NV>(v, is_max, head.wred[w]);
-    __syncthreads();
-    const unsigned tag = ++posts, set = tag & 1u;
-    if (w < NV) {
-      const bool mx = (is_max >> w) & 1u;
-      double r = head.wred[lane & (kClWarps - 1)][w];
-#pragma unroll
-      for (int o = kClWarps / 2; o > 0; o >>= 1) {
-        const double b = __shfl_xor_sync(kFull, r, o);
-        r = mx ? nanmax(r, b) : r + b;
-      }
-      const unsigned long long t = (unsigned long long)tag << 32;
-      if (lane < (int)size)
-        st_cluster_words(cluster_addr(smem_u32(&head.post[set][w][rank]), (unsigned)lane),
-                         t | (unsigned)__double2loint(r), t | (unsigned)__double2hiint(r));
-      ulonglong2 x = make_ulonglong2(0ull, 0ull);
-      unsigned spins = 0;
-      bool ready;
-      do {
-        if (lane < (int)size) x = ld_words(smem_u32(&head.post[set][w][lane]));
-        ready = lane >= (int)size || ((unsigned)(x.x >> 32) == tag && (unsigned)(x.y >> 32) == tag);
-      } while (!__all_sync(kFull, ready) && ++spins < kMaxPolls);
-      if (spins >= kMaxPolls && lane == 0) head.lost = 1;
-      r = lane < (int)size ? __hiloint2double((int)(unsigned)x.y, (int)(unsigned)x.x) : 0.0;
-#pragma unroll
-      for (int o = kMaxCluster / 2; o > 0; o >>= 1) {
-        const double b = __shfl_xor_sync(kFull, r, o);
-        r = mx ? nanmax(r, b) : r + b;
-      }
-      if (lane == 0) head.out[set][w] = r;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NV; ++q) out[q] = head.out[set][q];
-    return head.lost == 0;
-  }
 
   __device__ __forceinline__ void st_z(int c, int lane, const T (&v)[N]) const {
 #pragma unroll
@@ -498,7 +423,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
   const ClLayout<T> L(nb, (nb + (int)size - 1) / (int)size, S.rows);
   const int b0 = share(nb, rank, size), b1 = share(nb, rank + 1, size), nbl = b1 - b0;
   Cluster<T> C{M,
-               head,
+               ClusterTeam{head.posts, rank, size, 0u, 0u},
                Slots<T>{reinterpret_cast<T*>(g_cl_smem + L.slots), (nbl + CB - 1) / CB, b0, b1},
                reinterpret_cast<T*>(g_cl_smem + L.z),
                reinterpret_cast<double*>(g_cl_smem + L.y),
@@ -506,8 +431,6 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
                reinterpret_cast<const unsigned long long*>(g_cl_smem + L.mask),
                reinterpret_cast<const uint32_t*>(g_cl_smem + L.addr),
                reinterpret_cast<T*>(g_cl_smem + L.scratch + w * 512),
-               rank,
-               size,
                __ldg(M.xbase + b0),
                __ldg(M.xbase + b1),
                0,
@@ -516,8 +439,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
                reinterpret_cast<const T*>(g_cl_smem + L.rval),
                reinterpret_cast<const uint32_t*>(g_cl_smem + L.raddr),
                reinterpret_cast<const T*>(g_cl_smem + L.lval),
-               reinterpret_cast<const uint32_t*>(g_cl_smem + L.laddr),
-               0u};
+               reinterpret_cast<const uint32_t*>(g_cl_smem + L.laddr)};
   C.kept = min(C.r1 - C.r0, C.cap);
   const Slots<T>& K = C.K;
   const int nch = K.nch;
@@ -532,12 +454,8 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
       const unsigned k = (unsigned)(((long long)(b + 1) * size - 1) / nb);
       addr[b] = cluster_addr(zbase + (uint32_t)((b - share(nb, k, size)) * kBLEN * sizeof(T)), k);
     }
-    if (threadIdx.x == 0) {
-      head.nlong = 0u;
-      head.lost = 0;
-    }
-    for (int i = threadIdx.x; i < 2 * kRedMax * kMaxCluster; i += kClThreads)
-      (&head.post[0][0][0])[i] = make_ulonglong2(0ull, 0ull);  // no tag
+    if (threadIdx.x == 0) head.nlong = 0u;
+    head.posts.clear();
     if (MIXED && w == 0) {
       SineSolve<double> d;
       d.init();
@@ -581,7 +499,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
       }
     }
   }
-  cluster_sync();  // every CTA has started: its shared memory may be written
+  C.team.sync();  // every CTA has started: its shared memory may be written
   // the FP64 block solve of x = x + P^-1 y
   auto sine64 = [&]() {
     SineSolve<double> d;
@@ -597,19 +515,19 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
   };
   double* const row = reinterpret_cast<double*>(C.scratch);
   double mean_b = 0.0;
-  bool lost = false;  // a reduction gave up: the same for the CTA, which then leaves
+  bool lost = false;  // a wait ran out: the same for the cluster, which then leaves
   if constexpr (MIXED) {  // Neumann compatibility: project b to zero sum
     double v[1] = {0.0}, o[1];
     for (int blk = b0 + w; blk < b1; blk += kClWarps)
       v[0] += __ldg(V.b + blk * kBLEN + lane) + __ldg(V.b + blk * kBLEN + lane + 32);
-    lost = !C.reduce(v, 0u, o);
+    C.team.reduce(v, 0u, o);
     mean_b = o[0] / (double)(M.nb * kBLEN);
   }
   // r = b - A x (BiCGSTAB.cu:430-465)
   auto residual = [&](bool set_rh, double (&o)[6]) {
     ClResidual<T> epi{K, V.b, mean_b, set_rh, {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}};
     spmv_range<double>(M, V.x, b0, b1, C.r0, C.r1, epi, row);
-    lost = !C.reduce(epi.v, 0x23u, o) || lost;
+    C.team.reduce(epi.v, 0x23u, o);
   };
   double q[6];
   residual(true, q);
@@ -665,14 +583,15 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
         }
         zero_pnu = false;
       }
-      cluster_sync();
+      lost = !C.team.sync();
+      if (lost) break;
       // pass B: nu = A z; (rhat, nu)
       {
         ClRhNu<T> epi{K, 0.0};
         C.spmv(epi);
         const double v[1] = {epi.acc};
         double o[1];
-        lost = !C.reduce(v, 0u, o) || lost;
+        C.team.reduce(v, 0u, o);
         alpha = rho / (o[0] + eps);
       }
       // pass C: s = r - alpha nu (in place of r); z = P^-1 s
@@ -689,14 +608,15 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
           C.st_z(c, lane, sv);
         }
       }
-      cluster_sync();
+      lost = !C.team.sync();
+      if (lost) break;
       // pass D: t = A z; (t,s), (t,t)
       {
         ClTS<T> epi{K, 0.0, 0.0};
         C.spmv(epi);
         const double v[2] = {epi.ts, epi.tt};
         double o[2];
-        lost = !C.reduce(v, 0u, o) || lost;
+        C.team.reduce(v, 0u, o);
         omega = o[0] / (o[1] + eps);
       }
       // pass E: y += alpha p, y += omega s; r = s - omega t; norms; the
@@ -740,9 +660,9 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
                 make_double2(yv[2 * j], yv[2 * j + 1]);
         }
         if (threadIdx.x == 0 && globaltimer_ns() > deadline) v[4] = 1.0;
-        lost = !C.reduce(v, 0x11u, e) || lost;
+        C.team.reduce(v, 0x11u, e);
       }
-      if (e[4] != 0.0 || lost) {
+      if (e[4] != 0.0) {
         expired = true;
         break;
       }
@@ -764,7 +684,8 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
         if (claims || sqrt(nr) < sp.reliable_delta * rmax_since || since >= kMaxSweep) {
           since = 0;
           add_update(C, sine64(), V.x, V.xo, best_here);
-          cluster_sync();  // x before its neighbours read it
+          lost = !C.team.sync();  // x before its neighbours read it
+          if (lost) break;
           residual(sp.reliable_restart != 0, q);
           ++updates;
           refreshed = true;
@@ -806,9 +727,10 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
       }
     }
   }
-  if (expired || lost) {  // the deadline: the same in every CTA
+  // every way out of the loop, but for a lost wait, passes one more barrier:
+  // the wait that ran out may be the last reduction's
+  if (lost || !C.team.sync() || expired) {
     if (threadIdx.x == 0) atomicExch(S.abort_flag, 1);
-    cluster_sync();
     return;
   }
   // the solution: FP64 x0 + P^-1 y of the best y, mixed the best x; then its
@@ -835,7 +757,7 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
     hx[1] += 2.0 * (h * h);
   }
   double o[2] = {0.0, 1.0};
-  if (sp.subtract_mean && !C.reduce(hx, 0u, o) && threadIdx.x == 0) atomicExch(S.abort_flag, 1);
+  if (sp.subtract_mean) C.team.reduce(hx, 0u, o);
   const double avg = sp.subtract_mean ? o[0] / o[1] : 0.0;
   for (int lb = w; lb < nbl; lb += kClWarps) {
     double xv[2];
@@ -856,7 +778,8 @@ __device__ void cluster_solve(const ClusterArgs<T>& S) {
     s->err_opt = MIXED && status == CUP2D_OK ? err_true : err_opt;
     s->norm_ax0 = MIXED ? 0.0 : norm_ax0;
   }
-  cluster_sync();  // no CTA leaves while another may read its shared memory
+  // no CTA leaves while another may read its shared memory
+  if (!C.team.sync() && threadIdx.x == 0) atomicExch(S.abort_flag, 1);
 }
 
 __global__ void __launch_bounds__(kClThreads, 1) k_bicgstab64_cluster(const __grid_constant__ ClusterArgs<double> S) {

@@ -48,3 +48,21 @@ def test_team_reductions_are_ordered(tmp_path):
     exe = build(tmp_path, "team_threads.cpp", {"team.inc": ["common.cuh"]}, "-fsanitize=thread")
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "data race" not in r.stderr, r.stdout + r.stderr[:4000]
+
+
+# the reductions of the body in cluster_threads.cpp: 1 the mean, 2 the residual, then
+# B, D, E of an iteration (3 4 5, 6 7 8, 9 10 11), 12 the true residual, ..., 22 the last mean
+WAITS = [[0, 1], [2, 2], [0, 3], [2, 4], [0, 5], [2, 8], [1, 11], [0, 12], [2, 21], [0, 22], [1, 1, 2], [1, 7, 8]]
+
+
+def test_cluster_leaves_together(tmp_path):
+    """A CTA whose bounded wait ran out, in whichever reduction: all CTAs of the
+    cluster leave behind the same barrier, and none posts into the shared
+    memory of one that has left."""
+    inc = {"cluster.inc": ["common.cuh", "cluster_team.cuh"]}
+    runs = [(build(tmp_path, "cluster_threads.cpp", inc), [])]
+    (tmp_path / "short").mkdir()
+    short = build(tmp_path / "short", "cluster_threads.cpp", inc, "-DCUP2D_CLUSTER_POLLS=20")
+    for exe, args in runs + [(short, w) for w in WAITS]:
+        r = subprocess.run([str(exe), *map(str, args)], capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, (args, r.stdout, r.stderr)

@@ -100,3 +100,28 @@ def test_cluster_repeats_bit_for_bit(cuda):
         a = _solve(cuda, m, b, 0, tol_rel=1e-8, max_iter=5000, precision=precision)
         c = _solve(cuda, m, b, 0, tol_rel=1e-8, max_iter=5000, precision=precision)
         assert np.array_equal(a[0], c[0]) and a[1]["iterations"] == c[1]["iterations"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cluster_timeout(cuda, precision):
+    """The cluster kernel's own deadline: a 1 ms limit on a solve of some
+    hundred iterations (15 us each) to 1e-12.  The call reports it, and the
+    handle then solves as a fresh one does, bit for bit."""
+    import torch
+    from cup2d_b200 import Cup2dError
+    m = MESHES["sized_900"]()
+    b = torch.from_numpy(m.rhs_fourier(4)).to(cuda)
+    kw = dict(tol_rel=1e-8, max_iter=5000, precision=precision)
+    with Solver(m, tol_rel=1e-12, max_iter=100000, timeout_ms=1, precision=precision) as s:
+        for _ in range(2):
+            x = torch.zeros_like(b)
+            with pytest.raises(Cup2dError) as e:
+                s.solve_device(b, x)
+            assert e.value.status == L.TIMEOUT
+        s.set_opts(**kw)
+        x = torch.zeros_like(b)
+        assert s.solve_device(b, x)["status"] == L.OK
+    with Solver(m, **kw) as s:
+        y = torch.zeros_like(b)
+        assert s.solve_device(b, y)["status"] == L.OK
+    assert torch.equal(x, y)
