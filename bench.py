@@ -203,7 +203,8 @@ def spmv_leg(dev, stream, steps: int = 20, warmup: int = 5, forest: str = "full"
             out[name] = {"kernel": "k_apply", "ms": t, "bytes": by, "achieved": by / (t * 1e-3) / 1e9, "peak": peak,
                          "unit": "GB/s", "frac": by / (t * 1e-3) / 1e9 / peak, "peak_kind": kind,
                          "l2": "x and y larger than L2" if 2 * vb * n > 126e6 else "x and y fit in L2"}
-        # the mixed form's P^-1 apply alone, mma.sync (the solver's) and
+        # the mixed form's P^-1 apply alone, sine transforms on mma.sync (the
+        # solver's: four 8x8x8 products a block) and the dense 64x64 product on
         # tcgen05 (TMEM accumulators), on the same 73 M-cell vector: 8 B/cell
         g = torch.Generator(device=dev).manual_seed(2)
         p32 = torch.randn(n, dtype=torch.float32, device=dev, generator=g)
@@ -224,7 +225,7 @@ def spmv_leg(dev, stream, steps: int = 20, warmup: int = 5, forest: str = "full"
             out[name] = {"kernel": "k_precond32_tc" if tc else "k_precond32", "ms": t, "bytes": by,
                          "achieved": by / (t * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": by / (t * 1e-3) / 1e9 / peak, "peak_kind": kind,
-                         "flops_tensor_tflops": 3 * 2 * 64 * n / (t * 1e-3) / 1e12}
+                         "flops_tensor_tflops": 3 * 2 * (64 if tc else 32) * n / (t * 1e-3) / 1e12}
         del p32, z32, x, y
         # the pressure projection's field kernels on the same forest:
         # updatePressureRHS + updatePressureRHS1 (read vel, udef 16 B, chi,

@@ -61,7 +61,6 @@ namespace cup2d {
 
 namespace {
 
-constexpr int kPad = 68;  // staged block row (conflict-free fragment loads)
 constexpr int kMaxSweep = 64;  // mixed: longest FP32 sweep between true residuals
 
 // Shared memory of the solve kernels, per precision T of the Krylov vectors:
@@ -84,119 +83,6 @@ template <class T>
 __device__ __forceinline__ T* warp_scratch(Smem<T>& sm) { return spmv_stage(sm).z[0]; }
 template <class T>
 __device__ __forceinline__ double* spmv_row(Smem<T>& sm) { return reinterpret_cast<double*>(spmv_stage(sm).z[0]); }
-
-// P^-1 operand: FP64 rows, or the TF32 split of the FP32 P^-1 (hi, lo),
-// in rows of 64 values with the columns XOR-swizzled by the row (see the
-// Pinv specialisations): conflict-free fragment loads without padding.
-template <class T>
-struct PinvSmem;
-template <>
-struct PinvSmem<double> {
-  double v[kBLEN][kBLEN];
-};
-template <>
-struct PinvSmem<float> {
-  uint32_t hi[kBLEN][kBLEN];
-  uint32_t lo[kBLEN][kBLEN];
-};
-
-// ------------------------------------------------ P^-1 tile application ----
-
-template <class T>
-struct Pinv;
-
-// FP64: tiles of 8 blocks; warp w computes rows 8w..8w+7 with DMMA m8n8k4.
-// P^-1 stays in shared memory in rows of 64 doubles whose column c is stored
-// at c ^ 4*(r mod 8): the A-fragment loads (lane g,t reads row 8w+g, column
-// 4kk+t) hit every bank pair once per 16 lanes, the minimum two wavefronts
-// for 32 doubles.
-template <>
-struct Pinv<double> {
-  static constexpr int kTile = 8;
-  const double (*P)[kBLEN];
-  __device__ __forceinline__ static int swz(int r, int c) { return c ^ ((r & 7) << 2); }
-  // all threads; the caller synchronises before the first apply
-  __device__ __forceinline__ void load(PinvSmem<double>& s, const double* __restrict__ Pg, const float*) {
-    for (int q = threadIdx.x; q < kBLEN * kBLEN; q += blockDim.x) {
-      const int r = q / kBLEN, c = q % kBLEN;
-      s.v[r][swz(r, c)] = __ldg(Pg + q);
-    }
-    P = s.v;
-  }
-  __device__ __forceinline__ void apply(const double (*tile)[kPad], int w, int lane, int tb, int nvalid,
-                                        double* __restrict__ z) const {
-    const int g = lane >> 2, t = lane & 3;
-    const int r = 8 * w + g;  // r mod 8 == g
-    const double* arow = P[r];
-    double c0 = 0.0, c1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll
-    for (int kk = 0; kk < 16; kk += 2) {
-      dmma_884(c0, c1, arow[swz(r, 4 * kk + t)], tile[g][4 * kk + t]);
-      dmma_884(e0, e1, arow[swz(r, 4 * (kk + 1) + t)], tile[g][4 * (kk + 1) + t]);
-    }
-    c0 += e0;
-    c1 += e1;
-    if (2 * t < nvalid) z[(tb + 2 * t) * kBLEN + 8 * w + g] = c0;
-    if (2 * t + 1 < nvalid) z[(tb + 2 * t + 1) * kBLEN + 8 * w + g] = c1;
-  }
-};
-
-// FP32: tiles of 16 blocks; warp w computes rows 16*(w&3).. of blocks
-// 8*(w>>2).. with m16n8k8 TF32 MMA.  Operands are split x = hi + lo (both
-// TF32) and z = Phi*hi + Phi*lo + Plo*hi, accumulated in FP32, which keeps
-// the preconditioner apply at FP32 accuracy.  The split P = Phi + Plo (TF32
-// bit patterns) is formed once, in rows of 64 words whose column c is
-// stored at c ^ 4*(r mod 8): the A-fragment loads (lane g, t reads row
-// 16m+g, column 8kk+t) then fall in 32 distinct banks.
-template <>
-struct Pinv<float> {
-  static constexpr int kTile = 16;
-  const uint32_t (*Ph)[kBLEN];
-  const uint32_t (*Pl)[kBLEN];
-  __device__ __forceinline__ static int swz(int r, int c) { return c ^ ((r & 7) << 2); }
-  // all threads; the caller synchronises before the first apply
-  __device__ __forceinline__ void load(PinvSmem<float>& s, const double*, const float* __restrict__ P32) {
-    for (int q = threadIdx.x; q < kBLEN * kBLEN; q += blockDim.x) {
-      const int r = q / kBLEN, c = q % kBLEN;
-      const float v = __ldg(P32 + q);
-      const uint32_t hi = to_tf32(v);
-      s.hi[r][swz(r, c)] = hi;
-      s.lo[r][swz(r, c)] = to_tf32(v - __uint_as_float(hi));
-    }
-    Ph = s.hi;
-    Pl = s.lo;
-  }
-  __device__ __forceinline__ void apply(const float (*tile)[kPad], int w, int lane, int tb, int nvalid,
-                                        float* __restrict__ z) const {
-    const int g = lane >> 2, t = lane & 3, m = w & 3, nt = w >> 2;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* brow = tile[8 * nt + g];
-    const int ra = 16 * m + g, rb = ra + 8;  // ra mod 8 == rb mod 8: one swizzle for both
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const int c = 8 * kk + t;
-      const int c0 = swz(ra, c), c1 = swz(ra, c + 4);
-      const uint32_t ahi[4] = {Ph[ra][c0], Ph[rb][c0], Ph[ra][c1], Ph[rb][c1]};
-      const uint32_t alo[4] = {Pl[ra][c0], Pl[rb][c0], Pl[ra][c1], Pl[rb][c1]};
-      const float x0 = brow[c], x1 = brow[c + 4];
-      const uint32_t h0 = to_tf32(x0), h1 = to_tf32(x1);
-      const uint32_t l0 = to_tf32(x0 - __uint_as_float(h0)), l1 = to_tf32(x1 - __uint_as_float(h1));
-      mma_tf32(acc, alo, h0, h1);
-      mma_tf32(acc, ahi, l0, l1);
-      mma_tf32(acc, ahi, h0, h1);
-    }
-    const int n0 = 8 * nt + 2 * t, n1 = n0 + 1;
-    const int r0 = 16 * m + g, r1 = r0 + 8;
-    if (n0 < nvalid) {
-      z[(tb + n0) * kBLEN + r0] = acc[0];
-      z[(tb + n0) * kBLEN + r1] = acc[2];
-    }
-    if (n1 < nvalid) {
-      z[(tb + n1) * kBLEN + r0] = acc[1];
-      z[(tb + n1) * kBLEN + r1] = acc[3];
-    }
-  }
-};
 
 // ----------------------------------------------------- iteration core -----
 
@@ -1193,60 +1079,52 @@ cudaError_t launch_bicgstab_batch(const BatchArgs& a, int grid, bool mixed, cuda
 
 // ------------------------------------------------------- single ops -------
 
-__global__ void __launch_bounds__(kSolveThreads) k_precond64(const double* __restrict__ P, int nb,
-                                                             const double* __restrict__ p, double* __restrict__ z) {
-  __shared__ double tile[8][kPad];
-  __shared__ PinvSmem<double> Ps;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Pinv<double> pin;
-  pin.load(Ps, P, nullptr);
-  __syncthreads();
-  for (int tb = (int)blockIdx.x * 8; tb < nb; tb += (int)gridDim.x * 8) {
-    const int nvalid = (int)imin64(8, nb - tb);
-    if (w < nvalid) {
-      tile[w][lane] = p[(tb + w) * kBLEN + lane];
-      tile[w][lane + 32] = p[(tb + w) * kBLEN + lane + 32];
-    } else {
-      tile[w][lane] = 0.0;
-      tile[w][lane + 32] = 0.0;
-    }
-    __syncthreads();
-    pin.apply(tile, w, lane, tb, nvalid, z);
-    __syncthreads();
+// z = P^-1 p, the solve kernels' block solve alone, a warp a chunk.  p and z
+// need only their type's alignment.
+template <class T>
+__device__ __forceinline__ void precond_body(int nb, const T* p, T* z) {
+  constexpr int CB = Frag<T>::CB, N = Frag<T>::N;
+  __shared__ __align__(16) double scratch[kWarps][kBLEN];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nch = (nb + CB - 1) / CB;
+  SineSolve<T> pin;
+  pin.init();
+  for (int c = (int)blockIdx.x * kWarps + w; c < nch; c += (int)gridDim.x * kWarps) {
+    const int i0 = c * CB * kBLEN + Frag<T>::cell0(lane), nv = nb - c * CB;
+    T v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = j / 2 < nv ? p[i0 + (j / 2) * kBLEN + j % 2] : T(0);
+    pin.apply(v, reinterpret_cast<T*>(scratch[w]), lane);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (j / 2 < nv) z[i0 + (j / 2) * kBLEN + j % 2] = v[j];
   }
 }
 
-cudaError_t launch_precond64(const double* P, int64_t nb, const double* p, double* z, cudaStream_t s) {
+__global__ void __launch_bounds__(kSolveThreads) k_precond64(int nb, const double* p, double* z) {
+  precond_body<double>(nb, p, z);
+}
+__global__ void __launch_bounds__(kSolveThreads) k_precond32(int nb, const float* p, float* z) {
+  precond_body<float>(nb, p, z);
+}
+
+namespace {
+// CTAs for the chunks of nb blocks: enough to fill the device several times.
+template <class T>
+unsigned precond_grid(int64_t nb) {
+  constexpr int64_t per = kWarps * Frag<T>::CB;
+  return (unsigned)std::min<int64_t>((nb + per - 1) / per, 4096);
+}
+}  // namespace
+
+cudaError_t launch_precond64(int64_t nb, const double* p, double* z, cudaStream_t s) {
   if (nb <= 0) return cudaSuccess;
-  const int ctas = (nb + 7) / 8;
-  k_precond64<<<(unsigned)(ctas < 65535 ? ctas : 65535), kSolveThreads, 0, s>>>(P, nb, p, z);
+  k_precond64<<<precond_grid<double>(nb), kSolveThreads, 0, s>>>((int)nb, p, z);
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kSolveThreads) k_precond32(const float* __restrict__ P32, int nb,
-                                                             const float* __restrict__ p, float* __restrict__ z) {
-  __shared__ float tile[16][kPad];
-  __shared__ PinvSmem<float> Ps;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Pinv<float> pin;
-  pin.load(Ps, nullptr, P32);
-  __syncthreads();
-  for (int tb = (int)blockIdx.x * 16; tb < nb; tb += (int)gridDim.x * 16) {
-    const int nvalid = (int)imin64(16, nb - tb);
-    for (int j = w; j < 16; j += kWarps) {
-      tile[j][lane] = j < nvalid ? p[(tb + j) * kBLEN + lane] : 0.f;
-      tile[j][lane + 32] = j < nvalid ? p[(tb + j) * kBLEN + lane + 32] : 0.f;
-    }
-    __syncthreads();
-    pin.apply(tile, w, lane, tb, nvalid, z);
-    __syncthreads();
-  }
-}
-
-cudaError_t launch_precond32(const float* P32, int64_t nb, const float* p, float* z, cudaStream_t s) {
+cudaError_t launch_precond32(int64_t nb, const float* p, float* z, cudaStream_t s) {
   if (nb <= 0) return cudaSuccess;
-  const int ctas = (nb + 15) / 16;
-  k_precond32<<<(unsigned)(ctas < 65535 ? ctas : 65535), kSolveThreads, 0, s>>>(P32, nb, p, z);
+  k_precond32<<<precond_grid<float>(nb), kSolveThreads, 0, s>>>((int)nb, p, z);
   return cudaGetLastError();
 }
 

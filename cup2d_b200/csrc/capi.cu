@@ -65,35 +65,29 @@ cudaStream_t alloc_stream() {
   return t_alloc_stream[dev];
 }
 
-// P^-1 depends on nothing but the 8x8 block Laplacian: built once per
-// device (FP64, and rounded to FP32) and shared by every handle and batch.
-struct SharedPinv {
-  double* P = nullptr;
-  float* P32 = nullptr;
-};
-SharedPinv g_pinv[kMaxAllocDevices];
+// The dense P^-1 in FP32 (rounded from the FP64 build): it depends on nothing but
+// the 8x8 block Laplacian, so it is built once per device and shared by every
+// handle.
+float* g_pinv32[kMaxAllocDevices];
 
-int shared_pinv(const double** P, const float** P32) {
+int shared_pinv(const float** P32) {
   cudaStream_t s = alloc_stream();
   int dev = 0;
   if (!s || cudaGetDevice(&dev) != cudaSuccess) return CUP2D_CUDA_ERROR;
   std::lock_guard<std::mutex> g(g_alloc_mu);
-  SharedPinv& sp = g_pinv[dev];
-  if (!sp.P) {
+  if (!g_pinv32[dev]) {
     double* p = nullptr;
     float* p32 = nullptr;
     if (cudaMallocAsync(reinterpret_cast<void**>(&p), sizeof(double) * 4096, s) != cudaSuccess ||
         cudaMallocAsync(reinterpret_cast<void**>(&p32), sizeof(float) * 4096, s) != cudaSuccess ||
         launch_build_pinv(p, s) != cudaSuccess || launch_convert_f64_f32(p, p32, 4096, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
+        cudaFreeAsync(p, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
       cudaGetLastError();
       return CUP2D_CUDA_ERROR;
     }
-    sp.P = p;
-    sp.P32 = p32;
+    g_pinv32[dev] = p32;
   }
-  *P = sp.P;
-  *P32 = sp.P32;
+  *P32 = g_pinv32[dev];
   return CUP2D_OK;
 }
 
@@ -178,8 +172,7 @@ struct cup2d_poisson {
   DevBuf<unsigned long long> xmask;
   DevBuf<double> hblk, xval;
   DevBuf<float> xval32;
-  const double* P = nullptr;  // shared per device
-  const float* P32 = nullptr;
+  const float* P32 = nullptr;  // dense P^-1, shared per device
   DevBuf<int> err;
   DeviceMesh mesh;
   // Krylov vectors (FP64)
@@ -475,7 +468,7 @@ int handle_create(const cup2d_forest* forest, const cup2d_solve_opts* opts, cuda
   if (const char* e = std::getenv("CUP2D_GRID")) h->grid_override = std::atoi(e);
   // the no-allocation solve's static scratch is committed here, with the
   // rest of the handle's memory, so that those solves never load or allocate
-  if ((st = shared_pinv(&h->P, &h->P32)) || (st = ensure_scratch(h)) || (st = noalloc_prepare(h->device))) {
+  if ((st = shared_pinv(&h->P32)) || (st = ensure_scratch(h)) || (st = noalloc_prepare(h->device))) {
     cup2d_poisson_destroy(h);
     return st;
   }
@@ -883,13 +876,13 @@ int cup2d_poisson_transfer(const cup2d_poisson* src, const double* d_xsrc, const
 int cup2d_poisson_precond(cup2d_poisson* h, const double* d_p, double* d_z, void* stream) {
   if (!h || !d_p || !d_z) return CUP2D_INVALID_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the legacy default stream
-  return from_cuda(launch_precond64(h->P, h->nb, d_p, d_z, s));
+  return from_cuda(launch_precond64(h->nb, d_p, d_z, s));
 }
 
 int cup2d_poisson_precond32(cup2d_poisson* h, const float* d_p, float* d_z, void* stream) {
   if (!h || !d_p || !d_z) return CUP2D_INVALID_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the legacy default stream
-  return from_cuda(launch_precond32(h->P32, h->nb, d_p, d_z, s));
+  return from_cuda(launch_precond32(h->nb, d_p, d_z, s));
 }
 
 int cup2d_poisson_precond32_tc(cup2d_poisson* h, const float* d_p, float* d_z, void* stream) {

@@ -221,9 +221,10 @@ cudaError_t launch_bicgstab_batch(const BatchArgs& a, int grid, bool mixed, cuda
 // y = A x (spmv_apply.cu).
 cudaError_t launch_spmv64(const MeshView& M, const double* x, double* y, cudaStream_t s);
 cudaError_t launch_spmv32(const MeshView& M, const float* x, float* y, cudaStream_t s);
-cudaError_t launch_precond64(const double* P, int64_t nb, const double* p, double* z, cudaStream_t s);
-cudaError_t launch_precond32(const float* P32, int64_t nb, const float* p, float* z, cudaStream_t s);
-// The same apply on tcgen05 tensor cores with TMEM accumulators (precond_tc.cu).
+// z = P^-1 p as the solve kernels apply it (sine_solve.cuh).
+cudaError_t launch_precond64(int64_t nb, const double* p, double* z, cudaStream_t s);
+cudaError_t launch_precond32(int64_t nb, const float* p, float* z, cudaStream_t s);
+// The dense FP32 product on tcgen05 tensor cores with TMEM accumulators (precond_tc.cu).
 cudaError_t launch_precond32_tc(const float* P32, int64_t nb, const float* p, float* z, int* err, cudaStream_t s);
 
 // Forest of a handle on the device: per-block level and coordinates, and the

@@ -1,4 +1,4 @@
-// The mixed form's P^-1 apply (z = P^-1 p per 8x8 block, FP32 operands,
+// P^-1 as a dense product (z = P^-1 p per 8x8 block, FP32 operands,
 // split-TF32 accuracy) on the 5th-generation tensor cores: tcgen05.mma with
 // operands in shared memory and the accumulator in tensor memory (TMEM).
 // The role of the reference's cublasDgemm(T, N, 64, Nblocks, 64) with P_inv
@@ -19,9 +19,8 @@
 // K-halves of an 8-wide K step LBO = 128 bytes apart, 8-row groups SBO =
 // 2048 bytes apart (all 16 K-chunks of a row group are contiguous).
 //
-// The plain form of this apply is k_precond32 (mma.sync m16n8k8 TF32, the
-// one the solver's passes use); both are exported so that they can be timed
-// side by side.  A wait that outlives 2 s of globaltimer raises *err, and
+// The solver's passes apply P^-1 by sine transforms instead (sine_solve.cuh,
+// k_precond32 alone); both are exported so that they can be timed side by side.  A wait that outlives 2 s of globaltimer raises *err, and
 // the CTA still frees its tensor memory before leaving.
 #include <cuda_runtime.h>
 

@@ -33,7 +33,7 @@
 // 4 KB tile), and z comes out in the lanes that hold p.
 //
 // FP32: every product is split into TF32 terms, x = xh + xl, S = Sh + Sl,
-// X S = Xh Sh + Xl Sh + Xh Sl accumulated in FP32, as the dense form did.
+// X S = Xh Sh + Xl Sh + Xh Sl accumulated in FP32.
 #pragma once
 #include "common.cuh"
 #include "spmv.cuh"

@@ -258,9 +258,9 @@ class Solver:
                 "cup2d_poisson_transfer")
 
     def precond(self, p, z, stream=None, tcgen05: bool = False) -> None:
-        """z = P^-1 p per block: FP64, or FP32 (split TF32) on float32 tensors;
-        tcgen05=True takes the FP32 apply on the tcgen05 tensor cores (TMEM
-        accumulators) instead of mma.sync."""
+        """z = P^-1 p per block as the solves apply it: FP64, or FP32 (split
+        TF32) on float32 tensors; tcgen05=True takes the dense FP32 product on
+        the tcgen05 tensor cores (TMEM accumulators) instead."""
         if tcgen05:
             fn = L.lib().cup2d_poisson_precond32_tc
         else:

@@ -253,11 +253,12 @@ int cup2d_poisson_pressure_correction(cup2d_poisson* h, double dt, const double*
 int cup2d_poisson_pressure_projection(cup2d_poisson* h, double dt, double* d_vel, const double* d_udef,
                                       const double* d_chi, double* d_pres, double* d_pold, double* d_tmp,
                                       cup2d_solve_stats* stats, void* stream);
+/* z = P^-1 p per block as the FP64 solves apply it (sine transforms). */
 int cup2d_poisson_precond(cup2d_poisson* h, const double* d_p, double* d_z, void* stream);
-/* FP32 P^-1 apply of the mixed form (split-TF32 tensor-core MMA). */
+/* FP32 P^-1 apply of the mixed form (sine transforms, split-TF32 MMA). */
 int cup2d_poisson_precond32(cup2d_poisson* h, const float* d_p, float* d_z, void* stream);
-/* The same FP32 P^-1 apply on the 5th-generation tensor cores (tcgen05.mma,
- * accumulators in tensor memory): the cublasDgemm of P_inv
+/* FP32 P^-1 apply as one dense 64x64 product on the 5th-generation tensor cores
+ * (tcgen05.mma, accumulators in tensor memory): the cublasDgemm of P_inv
  * (source/Poisson/BiCGSTAB.cu:520,545) in the mixed form's precision,
  * measured beside cup2d_poisson_precond32.  Synchronises the stream;
  * CUP2D_TIMEOUT if the tensor-core work did not complete within 2 s. */
