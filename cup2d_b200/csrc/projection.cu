@@ -102,6 +102,7 @@ struct Geo {
       s.blk = c;
       return s;
     }
+#pragma unroll
     for (int h = 0; h < 2; ++h) {
       int64_t ci, cj;
       switch (f) {
@@ -118,50 +119,59 @@ struct Geo {
   }
 };
 
-// A field with `nc` doubles per cell.
+// Component c of a field with nc doubles per cell; vector: the component normal
+// to the face, whose sign a domain edge flips.
 struct Fld {
   const double* __restrict__ p;
-  int nc;
-  __device__ __forceinline__ double v(int64_t cell, int c) const { return p[cell * nc + c]; }
+  int nc, c;
+  bool vector;
+  __device__ __forceinline__ double v(int64_t cell) const { return p[cell * nc + c]; }
 };
 
-// Ghost of a fine cell (value vclose, next inward cell vfar) from coarse cell
-// (xc, yc) of block bc: ExpAMRSolver::interpolate on values.
-__device__ __noinline__ double interp_ghost(const Fld& w, int c, int64_t bc, int xc, int yc, double vclose, double vfar, double sT,
-                               bool xface) {
-  const int t = xface ? yc : xc;
-  auto cv = [&](int d) { return xface ? w.v(cidx(bc, xc, yc + d), c) : w.v(cidx(bc, xc + d, yc), c); };
-  double v0, v1, a0, a1, a2, b0, b1, b2;
-  const double v2 = cv(0);
-  if (t == kBS - 1 || t == kBS / 2 - 1) {
-    v0 = cv(-2); v1 = cv(-1);
-    a0 = 1. / 8.; a1 = -1. / 2.; a2 = 3. / 8.;
-    b0 = 1. / 32.; b1 = -1. / 16.; b2 = 1. / 32.;
-  } else if (t == 0 || t == kBS / 2) {
-    v0 = cv(2); v1 = cv(1);
-    a0 = -1. / 8.; a1 = 1. / 2.; a2 = -3. / 8.;
-    b0 = 1. / 32.; b1 = -1. / 16.; b2 = 1. / 32.;
-  } else {
-    v0 = cv(-1); v1 = cv(1);
-    a0 = -1. / 8.; a1 = 1. / 8.; a2 = 0.;
-    b0 = 1. / 32.; b1 = 1. / 32.; b2 = -1. / 16.;
+// Ghosts of fine cells from the coarse cell (xc, yc) of block bc:
+// ExpAMRSolver::interpolate on values.  The derivatives along the face are
+// those of the coarse cell; sT is the fine cell's side of its middle.
+struct Interp {
+  int64_t c0, c1, c2;
+  double a0, a1, a2, b0, b1, b2;
+  __device__ __forceinline__ Interp(int64_t bc, int xc, int yc, bool xface) {
+    const int t = xface ? yc : xc;
+    auto at = [&](int d) { return xface ? cidx(bc, xc, yc + d) : cidx(bc, xc + d, yc); };
+    const bool high = t == kBS - 1 || t == kBS / 2 - 1, low = t == 0 || t == kBS / 2;
+    c2 = at(0);
+    c0 = at(high ? -2 : low ? 2 : -1);
+    c1 = at(high ? -1 : 1);
+    a0 = high ? 1. / 8. : -1. / 8.;
+    a1 = high ? -1. / 2. : low ? 1. / 2. : 1. / 8.;
+    a2 = high ? 3. / 8. : low ? -3. / 8. : 0.;
+    b0 = 1. / 32.;
+    b1 = high || low ? -1. / 16. : 1. / 32.;
+    b2 = high || low ? 1. / 32. : -1. / 16.;
   }
-  const double d1 = (a0 * v0 + a1 * v1) + a2 * v2;
-  const double d2 = (b0 * v0 + b1 * v1) + b2 * v2;
-  const double tay = (v2 + sT * d1) + d2;
-  return (kI23 * vclose - kI15 * vfar) + kI815 * tay;
-}
+  __device__ __forceinline__ double ghost(double v0, double v1, double v2, double vclose, double vfar, double sT) const {
+    const double d1 = (a0 * v0 + a1 * v1) + a2 * v2;
+    const double d2 = (b0 * v0 + b1 * v1) + b2 * v2;
+    const double tay = (v2 + sT * d1) + d2;
+    return (kI23 * vclose - kI15 * vfar) + kI815 * tay;
+  }
+};
 
-// The ghost cell of one edge cell of block b across face f: one thread of the
-// block's lab fill (thread g of the block: face g / 8, cell g % 8 along it).
+// What a face cell needs of one field: its ghost (the lab value), and on a finer
+// face for the flux correction its own value, the two fine cells' and the ghosts
+// they see.
+struct FaceVals {
+  double g, own, fine[2], fine_ghost[2];
+};
+
+// The ghost cell of one edge cell of block b across face f: ghost gi of the
+// block (face gi / 8, cell gi % 8 along it).
 struct Ghost {
   const Geo& G;
   int64_t b, cell;
   int ix, iy, f;
   Side s;
 
-  // gi: the ghost's index in the block (face gi / 8); sd: the face's side,
-  // looked up by the caller ahead of its other loads
+  // sd: the face's side, looked up by the caller ahead of its other loads
   __device__ Ghost(const Geo& g, int64_t blk, int gi, const Side& sd) : G(g), b(blk), f(gi >> 3), s(sd) {
     const int k = gi & 7;
     ix = f == 0 ? 0 : f == 1 ? kBS - 1 : k;
@@ -171,45 +181,77 @@ struct Ghost {
   __device__ bool xface() const { return f < 2; }
   // fine block and the along-face position of the fine cells facing this cell
   __device__ void fine_cells(int64_t& fb, int& k0) const {
-    fb = s.fine[xface() ? (iy >= kBS / 2) : (ix >= kBS / 2)];
+    fb = (xface() ? iy : ix) >= kBS / 2 ? s.fine[1] : s.fine[0];
     k0 = ((xface() ? iy : ix) % (kBS / 2)) * 2;
   }
   // fine cell q (depth d), as a global cell index
   __device__ int64_t fine_cell(int64_t fb, int k0, int q, int d) const {
     return xface() ? mirror(f, fb, 0, k0 + q, d) : mirror(f, fb, k0 + q, 0, d);
   }
-  // The lab value of component c of field w in the ghost cell.
-  __device__ double value(const Fld& w, int c, bool vector) const {
-    switch (s.kind) {
-      case kSame:
-        return w.v(mirror(f, s.blk, ix, iy, 0), c);
-      case kEdge: {
-        const double own = w.v(cell, c);
-        return (vector && c == (xface() ? 0 : 1)) ? -own : own;
+  // The values of NF fields, all their loads ahead of the arithmetic.  One by one
+  // (a call per field, and per fine cell of a finer face) a warp of a block with
+  // coarse/fine faces waited for nine round trips in a row: us for the whole
+  // right-hand side 15.3 -> 6.6 on 128 blocks, 28.8 -> 12.7 on 6,000, correction 6.5 -> 3.6
+  // and 11.7 -> 5.9.
+  template <int NF>
+  __device__ __forceinline__ void values(const Fld (&w)[NF], FaceVals (&o)[NF]) const {
+    if (s.kind == kSame) {
+      const int64_t c = mirror(f, s.blk, ix, iy, 0);
+#pragma unroll
+      for (int k = 0; k < NF; ++k) o[k].g = w[k].v(c);
+    } else if (s.kind == kEdge) {
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        const double own = w[k].v(cell);
+        o[k].g = w[k].vector ? -own : own;
       }
-      case kCoarser: {
-        const int64_t bx = G.F.bx[b], by = G.F.by[b];
-        const int xc = f == 0 ? kBS - 1 : f == 1 ? 0 : (bx % 2 == 0 ? ix / 2 : ix / 2 + kBS / 2);
-        const int yc = f == 2 ? kBS - 1 : f == 3 ? 0 : (by % 2 == 0 ? iy / 2 : iy / 2 + kBS / 2);
-        const double sT = xface() ? (iy % 2 == 0 ? -1. : 1.) : (ix % 2 == 0 ? -1. : 1.);
-        const int64_t inward = cidx(b, ix + (f == 0 ? 1 : f == 1 ? -1 : 0), iy + (f == 2 ? 1 : f == 3 ? -1 : 0));
-        return interp_ghost(w, c, s.blk, xc, yc, w.v(cell, c), w.v(inward, c), sT, xface());
+    } else if (s.kind == kCoarser) {
+      const int64_t bx = G.F.bx[b], by = G.F.by[b];
+      const int xc = f == 0 ? kBS - 1 : f == 1 ? 0 : (bx % 2 == 0 ? ix / 2 : ix / 2 + kBS / 2);
+      const int yc = f == 2 ? kBS - 1 : f == 3 ? 0 : (by % 2 == 0 ? iy / 2 : iy / 2 + kBS / 2);
+      const double sT = xface() ? (iy % 2 == 0 ? -1. : 1.) : (ix % 2 == 0 ? -1. : 1.);
+      const int64_t inward = cidx(b, ix + (f == 0 ? 1 : f == 1 ? -1 : 0), iy + (f == 2 ? 1 : f == 3 ? -1 : 0));
+      const Interp I(s.blk, xc, yc, xface());
+      double v[NF][5];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        v[k][0] = w[k].v(I.c0);
+        v[k][1] = w[k].v(I.c1);
+        v[k][2] = w[k].v(I.c2);
+        v[k][3] = w[k].v(cell);
+        v[k][4] = w[k].v(inward);
       }
-      default: {
-        int64_t fb;
-        int k0;
-        fine_cells(fb, k0);
-        const double s00 = w.v(fine_cell(fb, k0, 0, 0), c), s01 = w.v(fine_cell(fb, k0, 1, 0), c);
-        const double s10 = w.v(fine_cell(fb, k0, 0, 1), c), s11 = w.v(fine_cell(fb, k0, 1, 1), c);
-        return 0.25 * ((s00 + s01) + (s10 + s11));
+#pragma unroll
+      for (int k = 0; k < NF; ++k) o[k].g = I.ghost(v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], sT);
+    } else {
+      int64_t fb;
+      int k0;
+      fine_cells(fb, k0);
+      const int64_t f00 = fine_cell(fb, k0, 0, 0), f01 = fine_cell(fb, k0, 1, 0);
+      const int64_t f10 = fine_cell(fb, k0, 0, 1), f11 = fine_cell(fb, k0, 1, 1);
+      // seen from the fine block, the interpolation is centred on this cell
+      const Interp I(b, ix, iy, xface());
+      double v[NF][7];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        v[k][0] = w[k].v(f00);
+        v[k][1] = w[k].v(f01);
+        v[k][2] = w[k].v(f10);
+        v[k][3] = w[k].v(f11);
+        v[k][4] = w[k].v(I.c0);
+        v[k][5] = w[k].v(I.c1);
+        v[k][6] = w[k].v(I.c2);
+      }
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        o[k].g = 0.25 * ((v[k][0] + v[k][1]) + (v[k][2] + v[k][3]));
+        o[k].own = v[k][6];
+        o[k].fine[0] = v[k][0];
+        o[k].fine[1] = v[k][1];
+        o[k].fine_ghost[0] = I.ghost(v[k][4], v[k][5], v[k][6], v[k][0], v[k][2], -1.);
+        o[k].fine_ghost[1] = I.ghost(v[k][4], v[k][5], v[k][6], v[k][1], v[k][3], 1.);
       }
     }
-  }
-  // Ghost of fine cell q of a finer face (seen from the fine block), the
-  // interpolation centred on this coarse cell.
-  __device__ double fine_ghost(const Fld& w, int c, int64_t fb, int k0, int q) const {
-    return interp_ghost(w, c, b, ix, iy, w.v(fine_cell(fb, k0, q, 0), c), w.v(fine_cell(fb, k0, q, 1), c),
-                        q == 0 ? -1. : 1., xface());
   }
 };
 
@@ -244,8 +286,10 @@ __device__ __forceinline__ double grad_face(int f, double pFac, double g, double
 // labs of one warp each were bound by the L1/shared-memory pipe (79-86 % busy,
 // lab rows and interleaved pairs conflicting).  us on 1.15 M blocks (73 M cells),
 // CTA labs -> warp labs -> shuffles: right-hand side and the reset of pres 1833
-// -> 1686 -> 1393 (3.4 TB/s), correction 1028 -> 724 -> 585 (5.0 TB/s); on 0.1 M blocks
-// 225 -> 206 -> 172 and 127 -> 89 -> 77.  Bound now by the ghosts' scattered sectors.
+// -> 1686 -> 1393, correction 1028 -> 724 -> 585; on 0.1 M blocks 225 -> 206 -> 172 and
+// 127 -> 89 -> 77.  With the ghosts' operands of all fields loaded together
+// (Ghost::values) 1139 (4.1 TB/s) and 462 (6.3 TB/s) on 1.15 M blocks.  Bound now by
+// the ghosts' scattered sectors.
 
 // The neighbours of a lane's two values a0 (cell l), a1 (cell l + 32): across
 // the block's faces the ghosts g of the other lanes.
@@ -301,10 +345,11 @@ struct FluxAt {
   }
 };
 
+// VEL, PRES: which of the two right-hand side parts the call asks for.
+template <bool VEL, bool PRES>
 __global__ void __launch_bounds__(kProjThreads, 3) k_pressure_rhs(const __grid_constant__ Geo G, double dt,
                                                                     const __grid_constant__ ProjFields P) {
   const int lane = threadIdx.x & 31;
-  const bool vel = P.vel != nullptr, pres = P.pres != nullptr;
   const int f = lane >> 3;
   const int64_t step = (int64_t)gridDim.x * kProjWarps;
   int64_t b = (int64_t)blockIdx.x * kProjWarps + (threadIdx.x >> 5);
@@ -315,29 +360,33 @@ __global__ void __launch_bounds__(kProjThreads, 3) k_pressure_rhs(const __grid_c
   }
   for (; b < G.F.nb; b += step) {
     const int64_t cell = b * kBLEN + lane;
-    const Fld V{P.vel, 2}, U{P.udef, 2}, Q{P.pres, 1};
     double2 u[2], ud[2];
     double chi[2], p[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      if (vel) {
+      if constexpr (VEL) {
         u[j] = __ldg(reinterpret_cast<const double2*>(P.vel) + cell + 32 * j);
         ud[j] = __ldg(reinterpret_cast<const double2*>(P.udef) + cell + 32 * j);
         chi[j] = __ldg(P.chi + cell + 32 * j);
       }
-      if (pres) p[j] = P.pres[cell + 32 * j];
+      if constexpr (PRES) p[j] = P.pres[cell + 32 * j];
     }
     const Ghost gh(G, b, lane, G.side_from_code(b, f, code));
     const unsigned finer = finer_faces(gh.s.kind);
     const double h = cell_h(G.F, level);
     const double facDiv = 0.5 * h / dt;
     const int cmp = gh.xface() ? 0 : 1;  // the normal component: the only one the divergence reads
-    double g = 0.0, gd = 0.0, gp = 0.0;
-    if (vel) {
-      g = gh.value(V, cmp, true);
-      gd = gh.value(U, cmp, true);
+    FaceVals v[3];  // vel, udef (VEL), pres (PRES)
+    if constexpr (VEL && PRES) {
+      const Fld w[3] = {{P.vel, 2, cmp, true}, {P.udef, 2, cmp, true}, {P.pres, 1, 0, false}};
+      gh.values(w, v);
+    } else if constexpr (VEL) {
+      const Fld w[2] = {{P.vel, 2, cmp, true}, {P.udef, 2, cmp, true}};
+      gh.values(w, reinterpret_cast<FaceVals(&)[2]>(v));
+    } else {
+      const Fld w[1] = {{P.pres, 1, 0, false}};
+      gh.values(w, reinterpret_cast<FaceVals(&)[1]>(v[2]));
     }
-    if (pres) gp = gh.value(Q, 0, false);
     // the next block's faces
     const int64_t bn = b + step;
     if (bn < G.F.nb) {
@@ -346,35 +395,35 @@ __global__ void __launch_bounds__(kProjThreads, 3) k_pressure_rhs(const __grid_c
     }
     double corr[2] = {0.0, 0.0};  // flux corrections: divergence, Laplacian
     if (gh.s.kind == kFiner) {
-      int64_t fb;
-      int k0;
-      gh.fine_cells(fb, k0);
-      if (vel) {
-        const double own = div_face(f, facDiv, __ldg(P.chi + gh.cell), g, V.v(gh.cell, cmp), gd, U.v(gh.cell, cmp));
-        const double facDivF = 0.5 * cell_h(G.F, G.F.level[fb]) / dt;
+      if constexpr (VEL) {
+        int64_t fb;
+        int k0;
+        gh.fine_cells(fb, k0);
+        const double chif[2] = {__ldg(P.chi + gh.fine_cell(fb, k0, 0, 0)), __ldg(P.chi + gh.fine_cell(fb, k0, 1, 0))};
+        const double own = div_face(f, facDiv, __ldg(P.chi + gh.cell), v[0].g, v[0].own, v[1].g, v[1].own);
+        const double facDivF = 0.5 * (0.5 * h) / dt;  // the finer blocks' h: half, exactly
         double fs[2];
-        for (int r = 0; r < 2; ++r) {
-          const int64_t fc = gh.fine_cell(fb, k0, r, 0);
-          fs[r] = div_face(f ^ 1, facDivF, __ldg(P.chi + fc), gh.fine_ghost(V, cmp, fb, k0, r), V.v(fc, cmp),
-                           gh.fine_ghost(U, cmp, fb, k0, r), U.v(fc, cmp));
-        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          fs[r] = div_face(f ^ 1, facDivF, chif[r], v[0].fine_ghost[r], v[0].fine[r], v[1].fine_ghost[r], v[1].fine[r]);
         corr[0] = own + (fs[0] + fs[1]);
       }
-      if (pres) {
-        const double own = gp - Q.v(gh.cell, 0);
+      if constexpr (PRES) {
+        const double own = v[2].g - v[2].own;
         double fs[2];
-        for (int r = 0; r < 2; ++r) fs[r] = gh.fine_ghost(Q, 0, fb, k0, r) - Q.v(gh.fine_cell(fb, k0, r, 0), 0);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) fs[r] = v[2].fine_ghost[r] - v[2].fine[r];
         corr[1] = own + (fs[0] + fs[1]);
       }
     }
     __syncwarp();
     double t[2];
-    if (vel) {
+    if constexpr (VEL) {
       Around a, d;
-      around_x(lane, u[0].x, u[1].x, g, a);
-      around_y(lane, u[0].y, u[1].y, g, a);
-      around_x(lane, ud[0].x, ud[1].x, gd, d);
-      around_y(lane, ud[0].y, ud[1].y, gd, d);
+      around_x(lane, u[0].x, u[1].x, v[0].g, a);
+      around_y(lane, u[0].y, u[1].y, v[0].g, a);
+      around_x(lane, ud[0].x, ud[1].x, v[1].g, d);
+      around_y(lane, ud[0].y, ud[1].y, v[1].g, d);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         t[j] = facDiv * ((a.e[j] - a.w[j]) + (a.n[j] - a.s[j]));
@@ -394,10 +443,10 @@ __global__ void __launch_bounds__(kProjThreads, 3) k_pressure_rhs(const __grid_c
       t[0] = P.tmp[cell];
       t[1] = P.tmp[cell + 32];
     }
-    if (pres) {
+    if constexpr (PRES) {
       Around a;
-      around_x(lane, p[0], p[1], gp, a);
-      around_y(lane, p[0], p[1], gp, a);
+      around_x(lane, p[0], p[1], v[2].g, a);
+      around_y(lane, p[0], p[1], v[2].g, a);
 #pragma unroll
       for (int j = 0; j < 2; ++j) t[j] -= ((a.w[j] + a.e[j]) + (a.s[j] + a.n[j])) - 4.0 * p[j];
       if (finer) {
@@ -422,7 +471,7 @@ __global__ void __launch_bounds__(kProjThreads, 4) k_pressure_correction(const _
                                                                            const double* __restrict__ pres,
                                                                            double* __restrict__ vel) {
   const int lane = threadIdx.x & 31;
-  const Fld Q{pres, 1};
+  const Fld Q[1] = {{pres, 1, 0, false}};
   const int f = lane >> 3;
   const int64_t step = (int64_t)gridDim.x * kProjWarps;
   int64_t b = (int64_t)blockIdx.x * kProjWarps + (threadIdx.x >> 5);
@@ -441,7 +490,9 @@ __global__ void __launch_bounds__(kProjThreads, 4) k_pressure_correction(const _
     const unsigned finer = finer_faces(gh.s.kind);
     const double h = cell_h(G.F, level);
     const double pFac = -0.5 * dt * h;
-    const double g = gh.value(Q, 0, false);
+    FaceVals q[1];
+    gh.values(Q, q);
+    const double g = q[0].g;
     const int64_t bn = b + step;
     if (bn < G.F.nb) {
       code = __ldg(G.nbr + 4 * bn + f);
@@ -449,14 +500,11 @@ __global__ void __launch_bounds__(kProjThreads, 4) k_pressure_correction(const _
     }
     double corr = 0.0;
     if (gh.s.kind == kFiner) {
-      const double own = grad_face(f, pFac, g, Q.v(gh.cell, 0));
-      int64_t fb;
-      int k0;
-      gh.fine_cells(fb, k0);
-      const double pFacF = -0.5 * dt * cell_h(G.F, G.F.level[fb]);
+      const double own = grad_face(f, pFac, g, q[0].own);
+      const double pFacF = -0.5 * dt * (0.5 * h);  // the finer blocks' h: half, exactly
       double fs[2];
-      for (int q = 0; q < 2; ++q)
-        fs[q] = grad_face(f ^ 1, pFacF, gh.fine_ghost(Q, 0, fb, k0, q), Q.v(gh.fine_cell(fb, k0, q, 0), 0));
+#pragma unroll
+      for (int r = 0; r < 2; ++r) fs[r] = grad_face(f ^ 1, pFacF, q[0].fine_ghost[r], q[0].fine[r]);
       corr = own + (fs[0] + fs[1]);
     }
     __syncwarp();
@@ -491,7 +539,7 @@ __global__ void __launch_bounds__(kProjThreads, 4) k_pressure_correction(const _
 
 // Persistent grid: the co-resident CTAs of a kernel (queried once per device).
 int persistent_grid(const void* fn, int which, int64_t ngroups) {
-  static std::atomic<int> cap[64][2];
+  static std::atomic<int> cap[64][4];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int g = cap[dev][which].load(std::memory_order_acquire);
@@ -511,16 +559,20 @@ int persistent_grid(const void* fn, int which, int64_t ngroups) {
 cudaError_t launch_pressure_rhs(const ForestView& F, const int32_t* nbr, double dt, const ProjFields& f,
                                 cudaStream_t s) {
   if (F.nb <= 0) return cudaSuccess;
-  const int grid = persistent_grid((const void*)k_pressure_rhs, 0, (F.nb + kProjWarps - 1) / kProjWarps);
+  const int which = (f.vel ? 2 : 0) + (f.pres ? 1 : 0);
+  if (which == 0) return cudaErrorInvalidValue;
+  auto* const fn = which == 3 ? k_pressure_rhs<true, true> : which == 2 ? k_pressure_rhs<true, false>
+                                                                        : k_pressure_rhs<false, true>;
+  const int grid = persistent_grid((const void*)fn, which, (F.nb + kProjWarps - 1) / kProjWarps);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
-  k_pressure_rhs<<<grid, kProjThreads, 0, s>>>(Geo{F, nbr}, dt, f);
+  fn<<<grid, kProjThreads, 0, s>>>(Geo{F, nbr}, dt, f);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pressure_correction(const ForestView& F, const int32_t* nbr, double dt, const double* pres,
                                        double* vel, cudaStream_t s) {
   if (F.nb <= 0) return cudaSuccess;
-  const int grid = persistent_grid((const void*)k_pressure_correction, 1, (F.nb + kProjWarps - 1) / kProjWarps);
+  const int grid = persistent_grid((const void*)k_pressure_correction, 0, (F.nb + kProjWarps - 1) / kProjWarps);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   k_pressure_correction<<<grid, kProjThreads, 0, s>>>(Geo{F, nbr}, dt, pres, vel);
   return cudaGetLastError();
