@@ -117,6 +117,7 @@ class Solver:
         L.check(L.lib().cup2d_poisson_set_opts(self._h, C.byref(self.opts)), "cup2d_poisson_set_opts")
 
     def set_grid(self, grid: int) -> None:
+        """CTAs of the grid kernels; 0: by size (small forests on one cluster)."""
         L.check(L.lib().cup2d_poisson_set_grid(self._h, int(grid)), "cup2d_poisson_set_grid")
 
     # ------------------------------------------------------------ solve ---
@@ -286,6 +287,7 @@ class Solver:
               "E: x, r, norms", "true residual", "mean removal", "sum b", "next problem")
 
     def set_profiling(self, enable: bool = True) -> None:
+        """Phase timers; solves run on the grid kernels while they are on."""
         L.check(L.lib().cup2d_poisson_set_profiling(self._h, int(bool(enable))), "set_profiling")
 
     def profile(self) -> dict:

@@ -136,7 +136,10 @@ int cup2d_poisson_update_mesh(cup2d_poisson* h, const cup2d_forest* forest);
  * built on the device (no host forest, one read-back of the block count)
  * and assembled as update_mesh does.  disks: host array of ndisks
  * (cx, cy, r) triples, ndisks <= 64.  *nblocks receives the new block count
- * (NULL to ignore).  Like update_mesh, it waits for the device first. */
+ * (NULL to ignore).  Like update_mesh, it waits for the device first.  The
+ * forest is built by one cooperative launch whose waits are bounded:
+ * CUP2D_TIMEOUT if it has not finished after 20 s, the handle's forest then
+ * unchanged. */
 int cup2d_poisson_adapt_disks(cup2d_poisson* h, int32_t ndisks, const double* disks, double band,
                               int64_t* nblocks);
 /* The handle's current forest, in the block order of its vectors: level and
@@ -145,8 +148,14 @@ int cup2d_poisson_adapt_disks(cup2d_poisson* h, int32_t ndisks, const double* di
 int cup2d_poisson_get_forest(const cup2d_poisson* h, int32_t* level, int32_t* bx, int32_t* by);
 int cup2d_poisson_set_opts(cup2d_poisson* h, const cup2d_solve_opts* opts);
 int64_t cup2d_poisson_num_cells(const cup2d_poisson* h);
-/* Number of CTAs of the persistent solve kernels (0 = size heuristic).  The
- * launch is clamped to what fits co-resident on the device. */
+/* Number of CTAs of the persistent solve kernels.  0 (the default): by size --
+ * a forest whose vectors fit the shared memory of one thread-block cluster (about
+ * 940 blocks in FP64, 1,650 in the mixed form) is solved by one cluster, a larger
+ * one on a grid of one CTA per 8 blocks.  An explicit grid selects the grid
+ * kernels at any size; it is clamped to what fits co-resident on the device.
+ * Mean-constrained solves, profiled solves (cup2d_poisson_set_profiling) and a
+ * server's always run on a grid.  The forms sum in different orders, so their
+ * iterates differ by rounding; each repeats itself bit for bit. */
 int cup2d_poisson_set_grid(cup2d_poisson* h, int32_t grid);
 int cup2d_poisson_destroy(cup2d_poisson* h);
 
@@ -270,7 +279,9 @@ int cup2d_poisson_export_csr(cup2d_poisson* h, int64_t* n, int64_t* nnz,
 /* Per-phase device timers (the counterpart of DeviceProfiler,
  * source/Utils/DeviceProfiler.cuh:26-108, compiled in with -DBICGSTAB_PROFILER
  * in the reference; here switched at run time).  While enabled, every solve
- * adds, per CTA, the time spent computing each phase and waiting at the grid
+ * runs on the grid kernels (the cluster kernel that solves small forests
+ * otherwise has no timers and takes a third to nine tenths of their time an
+ * iteration) and adds, per CTA, the time spent computing each phase and waiting at the grid
  * barrier that ends it.  cup2d_poisson_profile returns the per-CTA averages
  * in ms accumulated since enabling, for phases 0 residual / mean, 1 pass A
  * (p, P^-1), 2 pass B (SpMV), 3 pass C (x, s, P^-1), 4 pass D (SpMV),
