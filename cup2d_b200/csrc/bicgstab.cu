@@ -120,8 +120,8 @@ __device__ __forceinline__ bool computes_row(const MeshView& M, int row, int b0,
 
 // The vectors only their own CTA touches between true residuals, p and x, stay
 // in shared memory for as many of its chunks as fit: the passes of a large solve
-// run at the rate of L2 (8-11 TB/s), and p is 2 of pass A's 5 streams, x 2 of pass
-// E's 8.  On 20,834 blocks this measured FP64 48.5 -> 41.8 us, mixed 38.1 -> 36.5 us
+// wait for L2 (9 TB/s in FP64, 28 % of its peak), and p is 2 of pass A's 5 streams,
+// x 2 of pass E's 8.  On 20,834 blocks this measured FP64 48.5 -> 41.8 us, mixed 38.1 -> 36.5 us
 // an iteration.  A chunk of p is a slot of kSlotBytes (16 bytes a lane, the fragment
 // layout), a chunk of x CB slots in cell order.  p fills the slots first.
 constexpr int kSlotBytes = 512;

@@ -20,10 +20,11 @@
 // true-residual replacement (mixed).  So z and z2 share one buffer and neither
 // is read again after its SpMV.  y is FP64 in both forms.
 //
-// us an iteration, against the grid solver: FP64 128 blocks 18.5 -> 6.7, 449 17.9 ->
-// 9.2; mixed 128 19.0 -> 8.7, 1,502 19.8 -> 16.9.  What is left of one at 128 blocks
-// (13k clocks): 4.8k in the two SpMV passes (dependent shared loads), some 4.5k in
-// the three reductions, 2.4k in the block solves, 1.2k in the two barriers.
+// us an iteration, against the grid solver: FP64 128 blocks 17.1 -> 6.1, 449 17.1 ->
+// 8.3, 899 17.5 -> 14.5; mixed 128 18.8 -> 7.8, 1,499 19.7 -> 17.0.  What is left of one
+// at 128 blocks, in clocks when it took 6.7 us (13k): 4.8k in the two SpMV passes
+// (dependent shared loads), some 4.5k in the three reductions, 2.4k in the block
+// solves, 1.2k in the two barriers.
 //
 // Copies of the neighbours' blocks pushed ahead of each SpMV, so that no load
 // left the CTA, measured no faster (their stores cost what the loads had).
@@ -837,10 +838,13 @@ size_t cluster_limit(int device) {
 
 // The cluster solver takes every forest whose vectors fit (FP64 about 940
 // blocks, mixed 1,650), where it is still the faster one: us an iteration
-// against the grid solver, FP64 929 blocks 14.9 / 17.8, mixed 1,502 16.9 / 19.6.  Of
-// the cluster sizes the smallest with at most 12 blocks a CTA (with barriers in
-// place of the tagged reductions: FP64 65 blocks 9.7 / 7.7 / 6.2 / 6.6 us on 2 / 4 /
-// 8 / 16 CTAs, 128 blocks 9.8 / 7.6 / 7.3 on 4 / 8 / 16, 302 blocks 11.7 / 9.6 on 8 / 16).
+// against the grid solver, FP64 899 blocks 14.5 / 17.5, mixed 1,601 18.2 / 19.6, and
+// 10.6 / 17.9 on 575 blocks with 4,852 explicit rows.  Of the cluster sizes the
+// smallest with at most 12 blocks a CTA: past it twice the SMs give at most 7 % (us
+// in FP64 on 2 / 4 / 8 / 16 CTAs: 24 blocks 5.0 / 4.6 / 4.6 / 4.7, 48 blocks 6.5 / 5.0 / 4.7
+// / 4.8, 96 blocks 8.9 / 6.6 / 5.0 / 4.8, 128 refined - / 9.4 / 7.3 / 6.1, 302 on 8 / 16
+// 11.3 / 9.0; mixed 96 blocks 10.1 / 7.4 / 6.9 / 6.7), and several small solves share
+// the device.
 template <class T>
 int cluster_size(int device, int64_t nb) {
   const size_t most = cluster_limit(device);

@@ -48,9 +48,8 @@ constexpr int kRowBatch = 9;
 // sum_k vals[k] z[xcol[k]] of an explicit row, k ascending over [k0, k1).
 // The columns and values of the first kRowBatch entries are requested
 // together, then their gathers together (two dependent round trips for a
-// row of up to kRowBatch entries; coarse/fine rows hold 7-8); the rest of a
-// longer row follows in a plain loop.  The sum is accumulated in k order, as the
-// assembled row is.
+// row of up to kRowBatch entries); the rest of a longer row follows in a plain
+// loop.  The sum is accumulated in k order, as the assembled row is.
 template <class T>
 __device__ __forceinline__ T explicit_row(const MeshView& M, const T* __restrict__ z, int k0, int k1) {
   constexpr int W = kRowBatch<T>;

@@ -13,7 +13,8 @@
 // Bound by memory latency and the L2 reads of the halos' sectors; a CTA's warps
 // take consecutive blocks, so that most neighbours hit L1.  us on 1.15 M blocks,
 // one / two / four chunks a warp: FP64 267 / 237 / 230, FP32 182 / 125 / 142; on 0.1 M
-// blocks 41 / 39 / 40 and 26 / 26 / 25.  Tiles staged in shared memory by bulk copies
+// blocks 41 / 39 / 40 and 26 / 26 / 25.  Two for both types: four is 14 % behind in FP32,
+// and in FP64 3 % ahead on the larger forest and 3 % behind on the smaller.  Tiles staged in shared memory by bulk copies
 // with a CTA barrier a tile took 271 and 149, 46 and 31 (65 % of its time issuing).
 #include <cuda_runtime.h>
 
